@@ -79,22 +79,13 @@ void set_tuned_block(int law, int flux, int dim, int order, int precision, long 
 
 // Fused stage kernel or separate face and element kernels, per (law, flux,
 // element, order, precision, size bucket): the autotuner's measurement where
-// there is one, else the default below.  The default follows measurements on
-// B200 (128-thread tiles, 131k-180k triangles, 196k-663k tets; step time of
-// the separate kernels over the fused one): the fused kernel wins for the 2D
-// Euler (Roe, LLF), scalar and Maxwell laws at P2-P3 (1.10-1.45x), Euler P1
-// (1.08x) and P1 on tets (scalar P2: 1.11x, 1.21-1.38x); the separate kernels
-// win for Burgers (up to 1.56x), the exact Godunov flux, P4 on triangles (up to
-// 2x), the 3D Euler law and tets of higher order (1.07-1.43x), where the fused
-// tile's halo (rows read and faces evaluated by two tiles) and its larger
-// shared memory cost more than the face data the separate kernels pass
-// through device memory.
+// there is one, else the default below.
 std::map<std::tuple<int, int, int, int, int, int>, int> g_tune_fused;
 
 bool fused_default(int law, int flux, int dim, int order) {
-  if (law == DGP_LAW_BURGERS2D || law == DGP_LAW_EULER3D || flux == DGP_FLUX_GODUNOV) return false;
-  if (dim == 2) return order == 2 || order == 3 || (order == 1 && law == DGP_LAW_EULER2D);
-  return order == 1 || (law == DGP_LAW_SCALAR && order == 2);
+  (void)dim;
+  (void)order;
+  return !(law == DGP_LAW_EULER3D || flux == DGP_FLUX_GODUNOV);
 }
 
 bool tuned_fused(int law, int flux, int dim, int order, int precision, long long cells) {
@@ -272,100 +263,120 @@ static std::vector<int> morton_order(const HostMesh& m) {
   return order;
 }
 
-// Face records and halos of the fused stage kernel's tiles (TileMesh): for
-// tile t, every face with a side among its cells, in face order, with both
-// sides as local rows (own cells first, then the halo in order of first use)
-// and the face's FP64 normal and measure.  The fused kernel is built for the
-// solver (fused_ok) when every tile's halo fits in shared memory; whether the
-// stages then use it or the face and element kernels is tuned_fused's choice
-// (dgp_set_fused switches).
-static int build_tiles(dgp_solver s, int Etot, const std::vector<int>& fel, const std::vector<int>& fcode,
-                       const std::vector<double>& fnrm, const std::vector<double>& fj, const std::vector<int>& bpart,
-                       const std::vector<int>& cface) {
-  const int TE = s->ops.TE, nlf = s->tab.nlf, dim = s->b.dim;
+// Face records and halo sides of the fused stage kernel's tiles (TileMesh):
+// for tile t, every face with a side among its cells, in face order, and the
+// neighbours' sides of those faces (periodic partners included), sorted by
+// local face so that the kernel's warps contract one face's table rows.  The
+// fused kernel is built for the solver (fused_ok) when every tile's faces and
+// halo fit in shared memory; whether the stages then use it or the face and
+// element kernels is tuned_fused's choice (dgp_set_fused switches).
+template <int DIM>
+static int build_tiles_dim(dgp_solver s, int Etot, const std::vector<int>& fel, const std::vector<int>& fcode,
+                           const std::vector<double>& fnrm, const std::vector<double>& fj,
+                           const std::vector<int>& bpart, const std::vector<int>& cface) {
+  const int TE = s->ops.TE, nlf = s->tab.nlf;
   const int ntiles = (Etot + TE - 1) / TE;
-  std::vector<int> tf_off(1, 0), tf_side, tf_code, tf_bnd, th_off(1, 0), th_cell;
-  std::vector<double> tf_nrm, tf_fj;
-  std::vector<int> flist, halo;
-  int nh_max = 0;
+  // the tiles' faces and their halo sides' counts by local face (4: periodic
+  // partners)
+  struct Counts {
+    int halo[5];
+  };
+  std::vector<int> fl, foff(1, 0);
+  std::vector<Counts> counts(ntiles);
+  std::vector<int2> count(ntiles);
+  fl.reserve(fj.size() + fj.size() / 2);
+  foff.reserve(ntiles + 1);
+  int nh_max = 1, nf_max = 1;
   for (int t = 0; t < ntiles; ++t) {
     const int e0 = t * TE, e1 = std::min(e0 + TE, Etot);
-    flist.clear();
-    halo.clear();
+    const size_t f0 = fl.size();
     for (int e = e0; e < e1; ++e)
       for (int lf = 0; lf < nlf; ++lf) {
         const int k = cface[static_cast<size_t>(e) * nlf + lf];
-        if (k >= 0) flist.push_back(k);
+        if (k >= 0) fl.push_back(k);
       }
-    std::sort(flist.begin(), flist.end());
-    flist.erase(std::unique(flist.begin(), flist.end()), flist.end());
-    auto local = [&](int e) {
-      if (e >= e0 && e < e1) return e - e0;
-      for (size_t h = 0; h < halo.size(); ++h)
-        if (halo[h] == e) return TE + static_cast<int>(h);
-      halo.push_back(e);
-      return TE + static_cast<int>(halo.size()) - 1;
-    };
-    for (int k : flist) {
+    std::sort(fl.begin() + f0, fl.end());
+    fl.erase(std::unique(fl.begin() + f0, fl.end()), fl.end());
+    foff.push_back(static_cast<int>(fl.size()));
+    Counts c{};
+    int nh = 0;
+    for (size_t i = f0; i < fl.size(); ++i) {
+      const int k = fl[i];
       const int eL = fel[2 * static_cast<size_t>(k)], eR = fel[2 * static_cast<size_t>(k) + 1];
-      const int lL = local(eL);
-      const int ownL = (eL >= e0 && eL < e1) ? 1 : 0;
-      int side = lL, ownR = 0, kind = 0, bnd = -1;
-      if (eR >= 0) {
-        side |= (local(eR) + 1) << 16;
-        ownR = (eR >= e0 && eR < e1) ? 1 : 0;
-      } else {
-        bnd = -eR - 1;
-        if (bpart[bnd] >= 0) {
-          kind = 2;
-          side |= (local(bpart[bnd]) + 1) << 16;
-        } else {
-          kind = 1;
-        }
-      }
-      tf_side.push_back(side);
-      tf_code.push_back((fcode[k] & 0xfff) | (ownL << 12) | (ownR << 13) | (kind << 14));
-      tf_bnd.push_back(bnd);
-      for (int c = 0; c < dim; ++c) tf_nrm.push_back(fnrm[static_cast<size_t>(k) * dim + c]);
-      tf_fj.push_back(fj[k]);
+      if (eL < e0 || eL >= e1) ++c.halo[fcode[k] & 15], ++nh;
+      if (eR >= 0 ? (eR < e0 || eR >= e1) : bpart[-eR - 1] >= 0) ++c.halo[eR >= 0 ? (fcode[k] >> 4) & 15 : 4], ++nh;
     }
-    tf_off.push_back(static_cast<int>(tf_side.size()));
-    th_cell.insert(th_cell.end(), halo.begin(), halo.end());
-    th_off.push_back(static_cast<int>(th_cell.size()));
-    nh_max = std::max(nh_max, static_cast<int>(halo.size()));
+    counts[t] = c;
+    const int nf = static_cast<int>(fl.size() - f0);
+    count[t] = make_int2(nf, nh);
+    nh_max = std::max(nh_max, nh);
+    nf_max = std::max(nf_max, nf);
   }
-  s->fused_ok = s->ops.fused != nullptr && nh_max <= TE * nlf && s->ops.fused_smem(nh_max) + 8 * 1024 <= 227 * 1024;
+  s->fused_ok = s->ops.fused != nullptr && nlf * TE <= kHaloRef && bpart.size() < (1u << 26) &&
+                s->ops.fused_smem(nf_max, nh_max) + 4 * 1024 <= 227 * 1024;
   long long cells = 0;
   for (const auto& hm : s->meshes) cells += hm.E;
-  s->fused = s->fused_ok && tuned_fused(s->law, s->flux, dim, s->order, s->precision, cells);
+  s->fused = s->fused_ok && tuned_fused(s->law, s->flux, DIM, s->order, s->precision, cells);
   if (!s->fused_ok) return DGP_OK;
+  std::vector<FaceRec<DIM>> rec(static_cast<size_t>(ntiles) * nf_max);
+  std::vector<int2> th_side(static_cast<size_t>(ntiles) * nh_max, make_int2(-1, 0));
+  for (int t = 0; t < ntiles; ++t) {
+    const int e0 = t * TE, e1 = std::min(e0 + TE, Etot);
+    auto own = [&](int e) { return e >= e0 && e < e1; };
+    int place[5], nh = 0;
+    for (int c = 0; c < 5; ++c) {
+      place[c] = nh;
+      nh += counts[t].halo[c];
+    }
+    const size_t hbase = static_cast<size_t>(t) * nh_max;
+    auto halo = [&](int cell, int cls, int y) {
+      const int h = place[cls]++;
+      th_side[hbase + h] = make_int2(cell, y);
+      return kHaloRef | h;
+    };
+    for (int i = foff[t]; i < foff[t + 1]; ++i) {
+      const int k = fl[i];
+      const int eL = fel[2 * static_cast<size_t>(k)], eR = fel[2 * static_cast<size_t>(k) + 1];
+      const int lfL = fcode[k] & 15, lfR = (fcode[k] >> 4) & 15, perm = (fcode[k] >> 8) & 15;
+      FaceRec<DIM> r{};
+      unsigned side = own(eL) ? lfL * TE + (eL - e0) : halo(eL, lfL, lfL);
+      int kind = kFaceInterior, bnd = 0;
+      if (eR >= 0) {
+        side |= static_cast<unsigned>(own(eR) ? lfR * TE + (eR - e0) : halo(eR, lfR, lfR)) << 16;
+      } else {
+        bnd = -eR - 1;
+        kind = kFaceBoundary;
+        if (bpart[bnd] >= 0) {
+          kind = kFacePeriodic;
+          side |= static_cast<unsigned>(halo(bpart[bnd], 4, 4 | (bnd << 3))) << 16;
+        }
+      }
+      for (int c = 0; c < DIM; ++c) r.n[c] = fnrm[static_cast<size_t>(k) * DIM + c];
+      r.fj = fj[k];
+      r.side = static_cast<int>(side);
+      r.code = perm | (kind << 3) | (bnd << 5);
+      rec[static_cast<size_t>(t) * nf_max + (i - foff[t])] = r;
+    }
+  }
   TileMesh& tm = s->b.tm;
   int rc = DGP_OK;
-  int *d_tf_off, *d_tf_side, *d_tf_code, *d_tf_bnd, *d_th_off, *d_th_cell;
-  double *d_tf_nrm, *d_tf_fj;
-  if (th_cell.empty()) th_cell.push_back(0);
-  if (tf_side.empty()) {
-    tf_side.push_back(0);
-    tf_code.push_back(0);
-    tf_bnd.push_back(-1);
-    tf_fj.push_back(0.0);
-    tf_nrm.resize(dim, 0.0);
-  }
-  if ((rc = s->upload(&d_tf_off, tf_off)) || (rc = s->upload(&d_tf_side, tf_side)) ||
-      (rc = s->upload(&d_tf_code, tf_code)) || (rc = s->upload(&d_tf_bnd, tf_bnd)) ||
-      (rc = s->upload(&d_tf_nrm, tf_nrm)) || (rc = s->upload(&d_tf_fj, tf_fj)) ||
-      (rc = s->upload(&d_th_off, th_off)) || (rc = s->upload(&d_th_cell, th_cell)))
+  int2 *d_count, *d_th_side;
+  FaceRec<DIM>* d_rec;
+  if ((rc = s->upload(&d_count, count)) || (rc = s->upload(&d_rec, rec)) || (rc = s->upload(&d_th_side, th_side)))
     return rc;
-  tm.tf_off = d_tf_off;
-  tm.tf_side = d_tf_side;
-  tm.tf_code = d_tf_code;
-  tm.tf_bnd = d_tf_bnd;
-  tm.tf_nrm = d_tf_nrm;
-  tm.tf_fj = d_tf_fj;
-  tm.th_off = d_th_off;
-  tm.th_cell = d_th_cell;
+  tm.count = d_count;
+  tm.tf_rec = d_rec;
+  tm.th_side = d_th_side;
   tm.nh_max = nh_max;
+  tm.nf_max = nf_max;
   return DGP_OK;
+}
+
+static int build_tiles(dgp_solver s, int Etot, const std::vector<int>& fel, const std::vector<int>& fcode,
+                       const std::vector<double>& fnrm, const std::vector<double>& fj, const std::vector<int>& bpart,
+                       const std::vector<int>& cface) {
+  return s->b.dim == 2 ? build_tiles_dim<2>(s, Etot, fel, fcode, fnrm, fj, bpart, cface)
+                       : build_tiles_dim<3>(s, Etot, fel, fcode, fnrm, fj, bpart, cface);
 }
 
 // Builds the device state of a solver over the instances already in s->meshes
@@ -554,13 +565,16 @@ static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int fie
     for (size_t i = 0; i < t.phi.size(); ++i) phimax[i % np] = std::max(phimax[i % np], std::fabs(t.phi[i]));
     for (size_t i = 0; i < t.phif.size(); ++i) phimax[i % np] = std::max(phimax[i % np], std::fabs(t.phif[i]));
     if ((rc = s->upload_t(&b.phimax, phimax))) return rc;
+    s->stage_tab.resize(s->ops.stage_tab_bytes / 8 + 1);
+    s->ops.fill_stage_tab(t, phimax.data(), s->stage_tab.data());
+    b.htab = s->stage_tab.data();
   }
   {
     std::vector<double> blob(s->ops.blob_elems);
     s->ops.fill_blob(t.dphi.data(), t.phif.data(), t.phi.data(), t.qw.data(), blob.data());
     if ((rc = s->upload_t(&b.blob, blob))) return rc;
     std::vector<double> fblob(s->ops.fused_blob_elems, 0.0);
-    s->ops.fill_fused_blob(t.dphi.data(), t.phif.data(), t.phi.data(), t.qw.data(), fblob.data());
+    s->ops.fill_fused_blob(b.htab, fblob.data());
     if ((rc = s->upload_t(&b.fblob, fblob))) return rc;
     b.blob_bytes = static_cast<int>(s->ops.blob_elems * s->ops.tsize);
   }

@@ -127,6 +127,7 @@ struct dgp_solver_s {
   int graph_steps = 0;
   dgp::TimeCtl* h_ctl = nullptr;  // pinned, 2 entries
   LtsState lts;                    // local time stepping (off unless enabled)
+  std::vector<double> stage_tab;   // host storage of b.htab
   bool fused = false;              // stages run through the fused stage kernel
   bool fused_ok = false;           // the fused stage kernel is built for this solver
   bool tr_stale = false;           // the face-point traces (tr) lag the state (the fused

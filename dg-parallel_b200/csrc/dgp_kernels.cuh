@@ -66,9 +66,10 @@ struct Cfg {
   // shared memory per cell of a tile: FP64 state and u_n, G rows, face slots,
   // geometry, CFL eigenvalues
   static constexpr int CELL_BYTES = 16 * MNP + (int)sizeof(T) * (M * LDK + NS * M) + 8 * (NV + DIM * DIM + 1);
-  // shared-memory budget of a tile: 768 bytes per thread, at most 64 KB so
-  // that three tiles (with the table blob) share an SM whatever the order
-  static constexpr int SMEM_BUDGET = BLOCK * 768 < 64 * 1024 ? BLOCK * 768 : 64 * 1024;
+  // shared-memory budget of a tile of the element kernel: 768 bytes per
+  // thread, at most 96 KB so that two tiles (with the table blob) share an SM;
+  // up to P2 on tets and P4 on triangles every row thread then has a row
+  static constexpr int SMEM_BUDGET = BLOCK * 768 < 96 * 1024 ? BLOCK * 768 : 96 * 1024;
   static constexpr int TE_SMEM = SMEM_BUDGET / CELL_BYTES;
   static constexpr int TE_ROWS = BLOCK / M;
   static constexpr int TE = TE_SMEM < TE_ROWS ? (TE_SMEM < 1 ? 1 : TE_SMEM) : TE_ROWS;
@@ -156,24 +157,35 @@ struct DevTables {
   const double* eqw;   // nqe
   const double* ephi;  // nqe x NP
   double phi0;
+  int zero;  // 0
 };
 
-// Per-tile face records and halo lists of the fused stage kernel.  Tile t
+// One face of a tile in the fused stage kernel (read whole from shared
+// memory).  A side is an own side, (local face) * TE + local cell, or with
+// kHaloRef set the index of a halo side of the tile.
+constexpr int kHaloRef = 0x8000;
+constexpr int kFaceInterior = 0, kFaceBoundary = 1, kFacePeriodic = 2;
+template <int DIM>
+struct alignas(16) FaceRec {
+  double n[DIM];  // unit normal out of the left cell
+  double fj;      // |J_f|
+  int side;       // left side | right side (interior, periodic) << 16
+  int code;       // perm | kind << 3 | boundary face index (kinds 1, 2) << 5
+};
+
+// Per-tile face records and halo sides of the fused stage kernel.  Tile t
 // owns cells [t TE, (t + 1) TE); its faces are every face with a side in the
 // tile (a face between two tiles appears in both lists and is evaluated by
-// both, identically); a local row index l < TE is the own cell e0 + l, l >= TE
-// the halo cell th_cell[th_off[t] + l - TE].
+// both, identically).  A halo side is a neighbour's side of such a face, or a
+// periodic partner; sides are sorted by local face.
 struct TileMesh {
-  const int* tf_off;     // [ntiles + 1] face records of each tile
-  const int* tf_side;    // lL | (lR + 1) << 16 (interior) or (partner + 1) << 16 (periodic), 0 above
-  const int* tf_code;    // lfL | lfR << 4 | perm << 8 | ownL << 12 | ownR << 13 | kind << 14
-                         // (kind 0 interior, 1 boundary, 2 periodic)
-  const int* tf_bnd;     // boundary face index of kinds 1 and 2
-  const double* tf_nrm;  // [NTF][DIM] unit normal out of the left cell (FP64)
-  const double* tf_fj;   // [NTF] |J_f| (FP64)
-  const int* th_off;     // [ntiles + 1] halo cells of each tile
-  const int* th_cell;    // internal cell index of each halo row
-  int nh_max;            // largest halo of a tile
+  // both lists at a fixed pitch per tile, so that a tile's loads depend on no
+  // earlier one; unused halo entries have cell -1
+  const int2* count;    // [ntiles] face records, halo sides
+  const void* tf_rec;   // [ntiles][nf_max] FaceRec<DIM>
+  const int2* th_side;  // [ntiles][nh_max] (internal cell, local face; 4 | boundary face << 3 for a
+                        // periodic partner)
+  int nh_max, nf_max;   // largest counts of a tile
 };
 
 template <typename T>

@@ -570,6 +570,23 @@ __device__ __forceinline__ bool is_physical(const LawParams& lp, const T* Q) {
   }
 }
 
+// A sufficient condition for isPhysical without its division: density and
+// rho E - |m|^2 / 2 above zero by far more than the rounding of the pressure's
+// formula (false for infinities, NaN and states near the limits of T).  Only
+// states that fail it evaluate isPhysical.
+template <int LAW, typename T>
+__device__ __forceinline__ bool surely_physical(const LawParams& lp, const T* Q) {
+  if constexpr (LAW == DGP_LAW_EULER2D || LAW == DGP_LAW_EULER3D) {
+    constexpr T tol = sizeof(T) == 8 ? (T)1e-12 : (T)1e-5;
+    T m2 = Q[1] * Q[1] + Q[2] * Q[2];
+    if constexpr (LAW == DGP_LAW_EULER3D) m2 += Q[4] * Q[4];
+    const T re = Q[0] * Q[3];
+    return (lp.p[7] > 1.0) & (Q[0] > (T)1e-15) & (Q[0] < (T)1e15) & (re > ((T)0.5 + tol) * m2) & (re < (T)1e30);
+  } else {
+    return true;
+  }
+}
+
 // A sufficient condition for isPhysical at every point of a cell: each field
 // stays within B[j] of mean[j] (B from the modes k >= 1 and the largest basis
 // values), and density and pressure keep a relative margin far above the
@@ -588,7 +605,7 @@ __device__ __forceinline__ bool physical_bound(const LawParams& lp, const T* mea
       mm += m3 * m3;
     }
     const T e = mean[3] - B[3] - tol * (fabs(mean[3]) + B[3]);
-    return e - (T)0.5 * mm / rho * ((T)1 + tol) > (T)0;
+    return e * rho > (T)0.5 * mm * ((T)1 + (T)2 * tol);
   } else {
     return true;
   }

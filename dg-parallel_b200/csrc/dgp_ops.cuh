@@ -37,6 +37,7 @@ cudaError_t ops_prepare() {
   }
 
   if constexpr (adjoint_built<K>()) {
+    static_assert(adj_elem_smem<K>() <= kSmemPerCta - 1024, "adjoint element tile");
     const size_t as = adj_elem_smem<K>();
     if (as > 48 * 1024)
       return cudaFuncSetAttribute(adj_elem_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -137,8 +138,8 @@ void ops_stage(const DeviceBuffers& b, int stage, double time_factor, int fuse_c
 }
 
 template <class K>
-size_t ops_fused_smem(int nh_max) {
-  const size_t a = FusedSmem<K, false>::bytes(nh_max), b = FusedSmem<K, true>::bytes(nh_max);
+size_t ops_fused_smem(int nf_max, int nh_max) {
+  const size_t a = FusedSmem<K, false>::bytes(nf_max, nh_max), b = FusedSmem<K, true>::bytes(nf_max, nh_max);
   return a > b ? a : b;
 }
 
@@ -151,10 +152,12 @@ void ops_fused(const DeviceBuffers& b, const double* in, const double* u0, doubl
   a.Cout = out;
   a.U0out = u0copy;
   a.tab.blob = static_cast<const typename K::T*>(b.fblob);
+  const auto& tb = *static_cast<const StageTab<K>*>(b.htab);
+  const int nf = b.tm.nf_max, nh = b.tm.nh_max;
   const int grid = ops_grid_elem<K>(b.E);
   if constexpr (probe_built<K>()) {
     if (b.round_mask && !b.cell_inst) {
-      stage_kernel<K, false, false, true><<<grid, K::BLOCK, FusedSmem<K, false>::bytes(b.tm.nh_max), st>>>(a);
+      stage_kernel<K, false, false, true><<<grid, K::BLOCK, FusedSmem<K, false>::bytes(nf, nh), st>>>(a, tb);
       if (stage == 3) stage_finalize_kernel<K><<<1, kFinalizeThreads, 0, st>>>(a, grid);
       return;
     }
@@ -163,18 +166,18 @@ void ops_fused(const DeviceBuffers& b, const double* in, const double* u0, doubl
   if constexpr (FusedSmem<K>::UMMA_OK) tc = b.tensor_cores != 0;
   if (tc) {
     if constexpr (FusedSmem<K>::UMMA_OK) {
-      const size_t smem = FusedSmem<K, true>::bytes(b.tm.nh_max);
+      const size_t smem = FusedSmem<K, true>::bytes(nf, nh);
       if (b.cell_inst)
-        stage_kernel<K, true, true><<<grid, K::BLOCK, smem, st>>>(a);
+        stage_kernel<K, true, true><<<grid, K::BLOCK, smem, st>>>(a, tb);
       else
-        stage_kernel<K, false, true><<<grid, K::BLOCK, smem, st>>>(a);
+        stage_kernel<K, false, true><<<grid, K::BLOCK, smem, st>>>(a, tb);
     }
   } else {
-    const size_t smem = FusedSmem<K, false>::bytes(b.tm.nh_max);
+    const size_t smem = FusedSmem<K, false>::bytes(nf, nh);
     if (b.cell_inst)
-      stage_kernel<K, true, false><<<grid, K::BLOCK, smem, st>>>(a);
+      stage_kernel<K, true, false><<<grid, K::BLOCK, smem, st>>>(a, tb);
     else
-      stage_kernel<K, false, false><<<grid, K::BLOCK, smem, st>>>(a);
+      stage_kernel<K, false, false><<<grid, K::BLOCK, smem, st>>>(a, tb);
   }
   if (stage == 3) stage_finalize_kernel<K><<<1, kFinalizeThreads, 0, st>>>(a, ops_grid_elem<K>(b.E));
 }
@@ -353,6 +356,8 @@ Ops make_ops() {
   o.tsize = sizeof(typename K::T);
   o.blob_elems = ElemSmem<K>::blob_elems;
   o.fill_blob = &fill_table_blob<K>;
+  o.stage_tab_bytes = stage_tab_bytes<K>();
+  o.fill_stage_tab = &fill_stage_tab<K>;
   o.fill_fused_blob = &fill_fused_blob<K>;
   o.fused_blob_elems = FusedSmem<K>::fblob_elems;
   o.tensor_cores_ok = FusedSmem<K>::UMMA_OK;

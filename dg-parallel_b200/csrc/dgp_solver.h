@@ -33,7 +33,9 @@ struct DeviceBuffers {
   int* bpart = nullptr;
   void* bpphi = nullptr;
   void* blob = nullptr;   // element-kernel tables in shared-memory layout
-  void* fblob = nullptr;  // the fused stage kernel's tables (gradient rows in its G order)
+  void* fblob = nullptr;  // the fused stage kernel's tensor-core operand (its other tables are
+                          // kernel parameters: htab)
+  const void* htab = nullptr;  // host: StageTab of the instantiation, owned by the solver
   int blob_bytes = 0;
   void* phi = nullptr;
   void* dphi = nullptr;
@@ -178,7 +180,12 @@ struct Ops {
   // writes the element-kernel table blob (FP64) from dphi [KV][NP], phif [NS][NP],
   // phi [NQ][NP], qw [NQ]
   void (*fill_blob)(const double*, const double*, const double*, const double*, double*) = nullptr;
-  void (*fill_fused_blob)(const double*, const double*, const double*, const double*, double*) = nullptr;
+  // the fused stage kernel's parameter tables (StageTab, stage_tab_bytes of
+  // host memory; phimax: largest |phi_k| over volume and face points), and its
+  // tensor-core operand from them
+  size_t stage_tab_bytes = 0;
+  void (*fill_stage_tab)(const RefTables&, const double* phimax, void* out) = nullptr;
+  void (*fill_fused_blob)(const void* tab, double*) = nullptr;
   size_t fused_blob_elems = 0;
   bool tensor_cores_ok = false;  // the fused kernel has a tensor-core contraction for this shape
   bool probe_ok = false;         // the fused kernel has the rounding probe for this configuration
@@ -192,7 +199,7 @@ struct Ops {
   // the input rows in stage 1
   void (*fused)(const DeviceBuffers&, const double* in, const double* u0, double* out, double* u0copy, int stage,
                 double time_factor, int fuse_cfl, cudaStream_t) = nullptr;
-  size_t (*fused_smem)(int nh_max) = nullptr;
+  size_t (*fused_smem)(int nf_max, int nh_max) = nullptr;
   void (*cfl)(const DeviceBuffers&, cudaStream_t) = nullptr;
   void (*project)(const DeviceBuffers&, double t, cudaStream_t) = nullptr;
   // over cells [e_begin, e_end); lp: field parameters (nullptr: the solver's law)
