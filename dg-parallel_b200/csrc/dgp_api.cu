@@ -82,16 +82,22 @@ void set_tuned_block(int law, int flux, int dim, int order, int precision, long 
 // there is one, else the default below.
 std::map<std::tuple<int, int, int, int, int, int>, int> g_tune_fused;
 
-bool fused_default(int law, int flux, int dim, int order) {
+// Step times on B200, separate over fused, 100k-180k cells: 1.3-2.6 everywhere
+// on triangles (1.06-1.25 with the exact Riemann solver, FP64), 1.8-2.1 on tets
+// -- but 0.6-0.7 for the exact Riemann solver on tets in FP64, whose faces
+// between two tiles (every third) the fused form evaluates twice at ~700
+// operations a point (mixed: 1.00-1.07).
+bool fused_default(int law, int flux, int dim, int order, int precision) {
+  (void)flux;
   (void)dim;
   (void)order;
-  return !(law == DGP_LAW_EULER3D || flux == DGP_FLUX_GODUNOV);
+  return !(law == DGP_LAW_EULER3D && precision == DGP_PRECISION_FP64);
 }
 
 bool tuned_fused(int law, int flux, int dim, int order, int precision, long long cells) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto it = g_tune_fused.find(std::make_tuple(law, flux, dim, order, precision, size_bucket(cells)));
-  return it == g_tune_fused.end() ? fused_default(law, flux, dim, order) : it->second != 0;
+  return it == g_tune_fused.end() ? fused_default(law, flux, dim, order, precision) : it->second != 0;
 }
 
 void set_tuned_fused(int law, int flux, int dim, int order, int precision, long long cells, bool fused) {

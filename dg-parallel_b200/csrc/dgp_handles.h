@@ -42,6 +42,8 @@ struct dgp_law_s {
     dgp::LawParams lp{};
     lp.field = field;
     for (int i = 0; i < DGP_NPARAMS; ++i) lp.p[i] = p[i];
+    lp.ginv = 1.0 / p[7];
+    lp.gc4 = 2.0 / (p[7] - 1.0);
     lp.nbc = nbc;
     for (int i = 0; i < nbc; ++i) {
       lp.bc_id[i] = bc_id[i];

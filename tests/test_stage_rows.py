@@ -96,3 +96,35 @@ def test_periodic_partner_rows_match_oracle(tmp_path, order):
     s.step(0.0, dt)
     o.step(0.0, dt)
     assert rel(s.get_state(), o.state()) < 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("kind,jump", [("godunov", 1e-3), ("godunov", 1.0), ("euler3d", 0.1), ("euler3d", 1.0)])
+def test_exact_riemann_of_random_jumps_matches_oracle(tmp_path, kind, jump, fused):
+    """Piecewise constant states with jumps of every size between neighbours:
+    weak waves take riemann_face's short path, strong ones the full iteration.
+    The flux is the oracle's to rounding, so the right-hand side is to 1e-11."""
+    dim = 3 if kind == "euler3d" else 2
+    law, flux, field, prm, box = LAWS["euler3d"] if dim == 3 else \
+        (dgp.LAW_EULER2D, dgp.FLUX_GODUNOV, dgp.FIELD_VORTEX, VORTEX, 10.0)
+    msh = str(tmp_path / "m.msh")
+    meshgen.write_msh_v1(_mesh(kind, 129, box), msh)
+    o = Oracle(msh, law, flux, 0, field, prm)
+    s = dgp.Solver(dgp.Mesh.from_msh(msh), dgp.Law(law, flux, field, prm), 0)
+    s.set_fused(fused)
+    rng = np.random.default_rng(11)
+    u = o.state()
+    n = len(u)
+    phi0 = np.sqrt(2.0 if dim == 2 else 6.0)
+    rho, pr = np.exp(0.5 * jump * rng.normal(size=n)), np.exp(jump * rng.normal(size=n))
+    v = 0.3 + 0.8 * jump * rng.normal(size=(n, dim))
+    u[:, 0, 0] = rho
+    u[:, 1, 0], u[:, 2, 0] = rho * v[:, 0], rho * v[:, 1]
+    if dim == 3:
+        u[:, 4, 0] = rho * v[:, 2]
+    u[:, 3, 0] = pr / 0.4 + 0.5 * rho * (v ** 2).sum(axis=1)
+    u /= phi0
+    o.set_state(u)
+    s.set_state(u)
+    assert rel(s.rhs(0.1), o.rhs(0.1)) < 1e-11
