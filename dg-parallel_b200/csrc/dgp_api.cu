@@ -1262,14 +1262,30 @@ int dgp_run(dgp_solver s, double t0, double tend, double cfl, int max_steps, dou
   if (int rc = reset_probe_recorders(s)) return rc;
   s->ops.cfl(s->b, s->stream);
   DGP_CUDA(cudaGetLastError());
+  // Graphs are queued without a host round trip in between as far as the end
+  // of the run cannot lie (a step limit exactly, an end time by the last known
+  // step, three quarters of it), at most kAhead of them; then the status is read.
+  constexpr int kAhead = 8;
   TimeCtl c{};
+  long long queued = 0;  // steps
   for (long long guard = 0;; ++guard) {
-    const bool one = tail && max_steps - c.steps < K;
-    DGP_CUDA(cudaGraphLaunch(one ? s->graph1 : s->graph, s->stream));
+    long long left = max_steps > 0 ? max_steps - queued : (1LL << 40);
+    if (tend > 0) {
+      const double est = c.dt > 0 ? 0.75 * (tend - c.t) / c.dt : 1.0;
+      left = std::min(left, std::max(static_cast<long long>(std::min(est, 1e9)), 1LL));
+    }
+    int n = static_cast<int>(std::min<long long>(left / K, kAhead));
+    const bool ones = tail && left == max_steps - queued && n < kAhead;
+    if (n == 0 && !ones) n = 1;
+    for (int i = 0; i < n; ++i) DGP_CUDA(cudaGraphLaunch(s->graph, s->stream));
+    queued += static_cast<long long>(n) * K;
+    if (ones)
+      for (; queued < max_steps; ++queued) DGP_CUDA(cudaGraphLaunch(s->graph1, s->stream));
     if (int rc = read_ctl(s, &c)) return rc;
     if (c.done) break;
     if (!std::isfinite(c.dt) || !(c.dt > 0))
       return fail(DGP_ERR_NONPHYSICAL, "time step is not positive and finite");
+    queued = c.steps;
   }
   if (t_out) *t_out = c.t;
   if (steps_out) *steps_out = c.steps;

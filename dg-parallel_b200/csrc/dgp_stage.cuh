@@ -352,6 +352,13 @@ __device__ __forceinline__ void st_row(double* p, const double (&v)[N]) {
   }
 }
 
+// programmatic dependent launch: the next kernel of the stream may start its
+// CTAs as these leave room (and read what no kernel of the chain writes);
+// pdl_wait returns when the previous kernels have ended and their writes are
+// visible.  Without the launch attribute both do nothing.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
@@ -576,39 +583,30 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
   T* sBnd = reinterpret_cast<T*>(smem_raw + FS::oP(nfm, nhm));
   unsigned char* s_mark = smem_raw + FS::oM(nfm, nhm);
 
-  // Everything that the tile reads from global memory is requested here,
-  // before anything is waited for.  Bulk copies on one mbarrier: the own rows
-  // (where their bytes are whole 16-byte units: not at a last tile with an odd
-  // number of values, nor from a base on an odd 8 bytes, a stored state of an
-  // odd length), the face records, B of the tensor cores.  A bound on the
-  // first wait (a.mbar_polls) counts polls from their issue.
+  // What the tile reads from global memory is requested here, before anything
+  // is waited for; the solver's constant data even before the previous kernel
+  // of the stream has ended (pdl_wait).  Bulk copies on one mbarrier: the face
+  // records, the own rows (where their bytes are whole 16-byte units: not at a
+  // last tile with an odd number of values, nor from a base on an odd 8 bytes,
+  // a stored state of an odd length), B of the tensor cores.  A bound on the
+  // first wait (a.mbar_polls) counts polls from the rows' issue.
+  pdl_trigger();
   const int nrow = min(TE, a.mesh.E - e0);
   const bool bulk = FS::bulk_rows && (nrow * MNP) % 2 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
+  const uint32_t rb = bulk ? (uint32_t)(nrow * MNP * 8) : 0u;
   bool failed = false;
   if (tid == 0) {
     mbar_init(&bar, 1);
     if constexpr (FS::UMMA) mbar_init(&mma_bar, 1);
     const uint32_t fb = (uint32_t)(nfm * sizeof(FaceRec<DIM>));
-    const uint32_t rb = bulk ? (uint32_t)(nrow * MNP * 8) : 0u;
     mbar_arrive_expect_tx(&bar, fb + rb + (FS::UMMA ? (uint32_t)(2 * FS::b_bytes) : 0));
-    if (bulk) bulk_g2s(sRow, a.C + (size_t)e0 * MNP, rb, &bar);
     bulk_g2s(smem_raw + FS::oF, static_cast<const FaceRec<DIM>*>(a.tm.tf_rec) + (size_t)tile * nfm, fb, &bar);
     if constexpr (FS::UMMA) bulk_g2s(smem_raw + FS::oB, a.tab.blob, (uint32_t)(2 * FS::b_bytes), &bar);
-    if (a.mbar_polls > 0 && !mbar_test_polls(&bar, 0, a.mbar_polls)) failed = true;
   }
   // the thread's first halo side
   int2 hs = make_int2(-1, 0);
   if (tid < nhm * M) hs = ld_pinned_i2(a.tm.th_side + (size_t)tile * nhm + tid / M);
-  const int all_done = a.gctl->done;
-  const int2 cnt = a.tm.count[tile];
-  TimeCtl* c = a.ctl;
-  int inst = 0, eend = a.mesh.E, inst_done = 0;
-  if constexpr (ENS) {  // the tile belongs to one instance
-    inst = a.cell_inst[e0];
-    c = a.ctl + inst;
-    eend = a.inst_end[inst];
-    inst_done = c->done;
-  }
+  const int2 cnt = ld_pinned_i2(a.tm.count + tile);
   for (int i = tid; i < nrow * DIM * DIM; i += NT) {
     if constexpr (sizeof(T) == 8)
       cp_async8(sJi + i, a.mesh.jinv + (size_t)e0 * DIM * DIM + i);
@@ -621,15 +619,27 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
   double csz = 0.0;
   if (!state_dependent_speed(K::LAW) && a.stage == 3 && a.fuse_cfl && tid < nrow)
     csz = ld_pinned(a.mesh.csize + e0 + tid);
-  const double dt = c->dt;
+  if (tid < NQF) s_fqw[tid] = tb.fqw[tid];
+  if constexpr (PHYS)
+    for (int i = tid; i < TE + nhm; i += NT) s_mark[i] = 0;
+  int inst = 0, eend = a.mesh.E;
+  if constexpr (ENS) {  // the tile belongs to one instance
+    inst = a.cell_inst[e0];
+    eend = a.inst_end[inst];
+  }
   if constexpr (FS::UMMA) {
     // 32 columns of tensor memory for D, freed on every way out of the kernel
     if (tid < 32) tmem_alloc(&s_tmem, 32);
     tc_fence_before();
   }
-  if (tid < NQF) s_fqw[tid] = tb.fqw[tid];
-  if constexpr (PHYS)
-    for (int i = tid; i < TE + nhm; i += NT) s_mark[i] = 0;
+  pdl_wait();
+  if (tid == 0) {
+    if (bulk) bulk_g2s(sRow, a.C + (size_t)e0 * MNP, rb, &bar);
+    if (a.mbar_polls > 0 && !mbar_test_polls(&bar, 0, a.mbar_polls)) failed = true;
+  }
+  TimeCtl* c = a.ctl + inst;
+  const int all_done = a.gctl->done, inst_done = ENS ? c->done : 0;
+  const double dt = c->dt;
   __syncthreads();  // the barrier's initialisation
   if (all_done || inst_done) {
     // nothing to do: leave once the copies have landed
@@ -675,13 +685,13 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
           for (int k = 0; k < NP; ++k) cr[k] = (T)v[k];
         } else {
 #pragma unroll
-          for (int k = 0; k < NP; ++k) cr[k] = (T)__ldg(a.C + gbase + k);
+          for (int k = 0; k < NP; ++k) cr[k] = (T)a.C[gbase + k];
         }
       }
     } else if (live) {
       const bool drop = PHYS && s_mark[cell];
 #pragma unroll
-      for (int k = 0; k < NP; ++k) cr[k] = (k > 0 && drop) ? (T)0 : (T)__ldg(a.C + gbase + k);
+      for (int k = 0; k < NP; ++k) cr[k] = (k > 0 && drop) ? (T)0 : (T)a.C[gbase + k];
     }
     if (live) {
       own_points<K, RND, !FS::VREG>(tb, cr, sS, sV, prow, a.round_mask);
@@ -1070,26 +1080,36 @@ template <class K>
 __global__ void __launch_bounds__(kFinalizeThreads) stage_finalize_kernel(
     const __grid_constant__ StageArgs<typename K::T> a, int ntiles) {
   constexpr int NT = kFinalizeThreads;
-  __shared__ double red[NT / 32];
+  __shared__ double red[NT / 32], redd[NT / 32];
+  pdl_trigger();
+  pdl_wait();
   if (a.gctl->done) return;
   const double* part = a.partials;
   const double* dtp = a.partials + ntiles;
   const int tid = threadIdx.x;
   if (a.cell_inst) {
-    for (int i = tid; i < a.ninst; i += NT) {
+    // a warp per instance (a thread each took a round trip per few tiles)
+    for (int i = tid / 32; i < a.ninst; i += NT / 32) {
       TimeCtl* c = a.ctl + i;
       if (c->done) continue;
       double r = 0.0, d = 1e300;
-      for (int b = a.tile_first[i]; b < a.tile_first[i + 1]; ++b) {
+      for (int b = a.tile_first[i] + (tid & 31); b < a.tile_first[i + 1]; b += 32) {
         r += part[b];
         d = fmin(d, dtp[b]);
       }
-      c->resid = r;
-      c->t = c->t + c->dt;
-      c->steps += 1;
-      if (a.fuse_cfl) {
-        ctl_finalize(c, d);
-        if (c->done) c->t_mark_ns = device_clock_ns();
+      for (int o = 16; o > 0; o >>= 1) {
+        r += __shfl_xor_sync(0xffffffffu, r, o);
+        d = fmin(d, __shfl_xor_sync(0xffffffffu, d, o));
+      }
+      __syncwarp();
+      if ((tid & 31) == 0) {
+        c->resid = r;
+        c->t = c->t + c->dt;
+        c->steps += 1;
+        if (a.fuse_cfl) {
+          ctl_finalize(c, d);
+          if (c->done) c->t_mark_ns = device_clock_ns();
+        }
       }
     }
     __syncthreads();
@@ -1100,19 +1120,37 @@ __global__ void __launch_bounds__(kFinalizeThreads) stage_finalize_kernel(
     }
     return;
   }
+  // one round trip for the partials and the time control, one barrier
+  TimeCtl now;
+  if (tid == 0) now = *a.ctl;
   double r = 0.0, d = 1e300;
   for (int b = tid; b < ntiles; b += NT) {
     r += part[b];
     d = fmin(d, dtp[b]);
   }
-  r = block_sum<NT>(r, red);
-  d = block_min<NT>(d, red);
+  for (int o = 16; o > 0; o >>= 1) {
+    r += __shfl_xor_sync(0xffffffffu, r, o);
+    d = fmin(d, __shfl_xor_sync(0xffffffffu, d, o));
+  }
+  if ((tid & 31) == 0) {
+    red[tid >> 5] = r;
+    redd[tid >> 5] = d;
+  }
+  __syncthreads();
+  if (tid < 32) {
+    r = tid < NT / 32 ? red[tid] : 0.0;
+    d = tid < NT / 32 ? redd[tid] : 1e300;
+    for (int o = 16; o > 0; o >>= 1) {
+      r += __shfl_xor_sync(0xffffffffu, r, o);
+      d = fmin(d, __shfl_xor_sync(0xffffffffu, d, o));
+    }
+  }
   if (tid == 0) {
-    TimeCtl* c = a.ctl;
-    c->resid = r;
-    c->t = c->t + c->dt;
-    c->steps += 1;
-    if (a.fuse_cfl) ctl_finalize(c, d);
+    now.resid = r;
+    now.t = now.t + now.dt;
+    now.steps += 1;
+    if (a.fuse_cfl) ctl_finalize(&now, d);
+    *a.ctl = now;
   }
 }
 
