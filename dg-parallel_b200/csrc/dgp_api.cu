@@ -1165,6 +1165,7 @@ static void launch_step(dgp_solver s, int fuse_cfl) {
     double* X1 = static_cast<double*>(b.X1);
     double* X2 = static_cast<double*>(b.X2);
     DeviceBuffers bl = b;
+    if (s->limiter == DGP_LIMITER_MOMENT) bl.tr = nullptr;  // the fused form keeps no traces
     s->ops.fused(b, C, C, X1, nullptr, 1, 0.0, 0, s->stream);
     if (lim) {
       bl.C = X1;
@@ -1177,7 +1178,8 @@ static void launch_step(dgp_solver s, int fuse_cfl) {
     }
     s->ops.fused(b, X2, C, C, nullptr, 3, 0.5, lim ? 0 : fuse_cfl, s->stream);
     if (lim) {
-      s->ops.limit(b, 1, s->stream);
+      bl.C = C;
+      s->ops.limit(bl, 1, s->stream);
       if (fuse_cfl) s->ops.cfl(b, s->stream);
     }
     s->tr_stale = true;
@@ -1631,12 +1633,15 @@ int dgp_ensemble_get_state(dgp_ensemble e, int i, double* host_state) {
   if (!host_state) return fail(DGP_ERR_INVALID, "null argument");
   DGP_CUDA(cudaSetDevice(s->device));
   DGP_CUDA(cudaStreamSynchronize(s->stream));
-  const int E = s->meshes[k].E, off = s->inst_off[k], uf = s->inst_ufirst[k];
-  std::vector<double> tmp(static_cast<size_t>(E) * mnp);
-  DGP_CUDA(cudaMemcpy(tmp.data(), static_cast<double*>(s->b.C) + static_cast<size_t>(off) * mnp,
-                      tmp.size() * 8, cudaMemcpyDeviceToHost));
-  for (int r = 0; r < E; ++r)
-    std::memcpy(&host_state[static_cast<size_t>(s->i2f[off + r] - uf) * mnp], &tmp[r * mnp], mnp * 8);
+  // reordered on the device, then one copy into the caller's array
+  const int E = s->meshes[k].E;
+  const size_t n = static_cast<size_t>(E) * mnp;
+  double* stage = static_cast<double*>(s->b.scratch);
+  gather_cells<double, double><<<static_cast<int>((n + 255) / 256), 256, 0, s->stream>>>(
+      static_cast<const double*>(s->b.C), stage, s->d_f2i + s->inst_ufirst[k], E, static_cast<int>(mnp));
+  DGP_CUDA(cudaGetLastError());
+  DGP_CUDA(cudaMemcpyAsync(host_state, stage, n * 8, cudaMemcpyDeviceToHost, s->stream));
+  DGP_CUDA(cudaStreamSynchronize(s->stream));
   return DGP_OK;
 }
 
@@ -1708,22 +1713,33 @@ int dgp_ensemble_run(dgp_ensemble e, double t0, double tend, double cfl, int max
   if (!e || !(cfl > 0)) return fail(DGP_ERR_INVALID, "bad argument");
   if (tend <= 0 && max_steps <= 0) return fail(DGP_ERR_INVALID, "need an end time or a step count");
   const int G = static_cast<int>(e->groups.size());
+  // graphs of K steps; the last steps under a step limit go through one-step
+  // graphs (a finished instance's kernels return at once, but six such steps
+  // of four groups cost what two real ones do)
+  constexpr int K = 8;
+  const bool tail = max_steps > 0 && max_steps % K != 0;
+  long long queued = 0;
   dgp_solver s0 = e->groups[0];
   DGP_CUDA(cudaSetDevice(s0->device));
   for (dgp_solver s : e->groups) {
     // drain earlier work (set_state, project) before the controls change
     DGP_CUDA(cudaStreamSynchronize(s->stream));
-    if (!s->graph) {
-      const int K = 8;
+    auto capture = [&](int steps, cudaGraphExec_t* out) -> int {
       cudaGraph_t g;
       DGP_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-      for (int k = 0; k < K; ++k) launch_step(s, 1);
+      for (int k = 0; k < steps; ++k) launch_step(s, 1);
       DGP_CUDA(cudaStreamEndCapture(s->stream, &g));
-      cudaError_t err = cudaGraphInstantiate(&s->graph, g, 0);
+      cudaError_t err = cudaGraphInstantiate(out, g, 0);
       cudaGraphDestroy(g);
       if (err != cudaSuccess) return fail(DGP_ERR_CUDA, std::string("graph: ") + cudaGetErrorString(err));
+      return DGP_OK;
+    };
+    if (!s->graph) {
+      if (int rc = capture(K, &s->graph)) return rc;
       s->graph_steps = K;
     }
+    if (tail && !s->graph1)
+      if (int rc = capture(1, &s->graph1)) return rc;
     const int n = s->b.ninst;
     std::vector<TimeCtl> c(n + 1);
     for (auto& x : c) {
@@ -1751,10 +1767,21 @@ int dgp_ensemble_run(dgp_ensemble e, double t0, double tend, double cfl, int max
   for (int g = 0; g < G; ++g) gpin[g] = &e->groups[g]->h_ctl[1];
   for (;;) {
     int all = 1;
+    // with a step limit every graph up to it is known to be needed unless the
+    // end time comes first: at most four at once
+    int n = 1, ones = 0;
+    if (max_steps > 0) {
+      const long long left = max_steps - queued;
+      n = static_cast<int>(std::min<long long>(left / K, tend > 0 ? 1 : 4));
+      if (tail && n * K == left - left % K) ones = static_cast<int>(left % K);
+      if (n + ones == 0) n = 1;
+      queued += static_cast<long long>(n) * K + ones;
+    }
     for (int g = 0; g < G; ++g)
       if (!done[g]) {
         dgp_solver s = e->groups[g];
-        DGP_CUDA(cudaGraphLaunch(s->graph, s->stream));
+        for (int i = 0; i < n; ++i) DGP_CUDA(cudaGraphLaunch(s->graph, s->stream));
+        for (int i = 0; i < ones; ++i) DGP_CUDA(cudaGraphLaunch(s->graph1, s->stream));
         DGP_CUDA(cudaMemcpyAsync(gpin[g], s->b.gctl, sizeof(TimeCtl), cudaMemcpyDeviceToHost, s->stream));
       }
     for (int g = 0; g < G; ++g)

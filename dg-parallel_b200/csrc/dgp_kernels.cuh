@@ -225,6 +225,13 @@ struct StageArgs {
   int p0;          // 1: P0 fallback on (face kernel marks, element kernel consumes marks)
 };
 
+// programmatic dependent launch: the next kernel of the stream may start its
+// CTAs as these leave room (and read what no kernel of the chain writes);
+// pdl_wait returns when the previous kernels have ended and their writes are
+// visible.  Without the launch attribute both do nothing.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void flag_nonphysical(Status* st, int cell) {
   atomicAdd(&st->nonphysical, 1);
   atomicMin(&st->first_bad, cell);
@@ -649,6 +656,8 @@ template <class K>
 __global__ void __launch_bounds__(256) cfl_kernel(const __grid_constant__ StageArgs<typename K::T> a) {
   __shared__ double red[256 / 32];
   __shared__ bool amLast;
+  pdl_trigger();
+  pdl_wait();
   if (a.gctl->done) return;
   TimeCtl* c = a.ctl;
   int e = blockIdx.x * 256 + threadIdx.x, eend = a.mesh.E;

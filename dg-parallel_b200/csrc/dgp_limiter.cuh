@@ -42,14 +42,16 @@ constexpr double kLimSmall = 1.0e-10;
 
 struct LimArgs {
   double* C;            // state, limited in place
-  double* Mo;           // [E * M][NP] moments of every degree of each row of the unlimited state
+  double* Mo;           // [NP][E * M] moments of every degree of each row of the unlimited state:
+                        // mode-major, so that a warp's rows and their neighbours (close in the
+                        // Morton order) share sectors
   unsigned char* big;   // [E * M] bit n: a mode of degree n above kLimSmall in magnitude
   unsigned char* trig;  // [E * M] trigger degree of each row (0: untouched)
   const int* nb;        // [E][4] left, right, bottom, top (-1: none)
   const double* geo;    // [E][kLimGeo]
   const double* Dn;     // per degree n: (n+1)^2 block at n(n+1)(2n+1)/6
   const double* Dinv;
-  void* tr;             // face-point traces (slot layout, type of the right-hand side)
+  void* tr;             // face-point traces (slot layout, type of the right-hand side); nullptr: not kept
   const void* phif;     // [NS][NP] face-point basis values (same type)
   const TimeCtl* ctl;   // kernels are no-ops once the run is done (nullptr: always run)
   const TimeCtl* gctl;
@@ -163,10 +165,11 @@ __device__ __forceinline__ void lim_row_moments(const double* __restrict__ row, 
 template <class K>
 __global__ void __launch_bounds__(128) limit_moments_kernel(LimArgs a) {
   constexpr int M = K::M, NP = K::NP, P = K::ORDER;
-  // the CTA's 128 rows are contiguous in the state and in the moments: both
-  // move through shared memory with coalesced loads and stores
+  // the CTA's 128 rows are contiguous in the state: they come through shared
+  // memory with coalesced loads
   __shared__ double s[128 * NP];
-  __shared__ unsigned char s_act[128];
+  pdl_trigger();
+  pdl_wait();
   if (a.ctl && a.gctl->done) return;
   const size_t R = (size_t)a.E * M;
   const size_t r0 = blockIdx.x * (size_t)128;
@@ -175,26 +178,20 @@ __global__ void __launch_bounds__(128) limit_moments_kernel(LimArgs a) {
   for (int i = t; i < nr * NP; i += 128) s[i] = a.C[r0 * NP + i];
   __syncthreads();
   const size_t r = r0 + t;
-  bool active = t < nr;
-  const int e = active ? static_cast<int>(r / M) : 0;
-  if (active && lim_skip_cell(a, e)) active = false;
-  s_act[t] = active ? 1 : 0;
-  if (active) {
-    double gg[4];
+  if (t >= nr) return;
+  const int e = static_cast<int>(r / M);
+  if (lim_skip_cell(a, e)) return;
+  double gg[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) gg[i] = __ldg(a.geo + (size_t)e * kLimGeo + i);
-    double row[NP], mo[NP];
+  for (int i = 0; i < 4; ++i) gg[i] = __ldg(a.geo + (size_t)e * kLimGeo + i);
+  double row[NP], mo[NP];
 #pragma unroll
-    for (int k = 0; k < NP; ++k) row[k] = s[t * NP + k];
-    unsigned big = 0;
-    lim_row_moments<P, NP>(row, a.Dn, gg, mo, big);
+  for (int k = 0; k < NP; ++k) row[k] = s[t * NP + k];
+  unsigned big = 0;
+  lim_row_moments<P, NP>(row, a.Dn, gg, mo, big);
 #pragma unroll
-    for (int k = 0; k < NP; ++k) s[t * NP + k] = mo[k];  // the thread's own row
-    a.big[r] = static_cast<unsigned char>(big);
-  }
-  __syncthreads();
-  for (int i = t; i < nr * NP; i += 128)
-    if (s_act[i / NP]) a.Mo[r0 * NP + i] = s[i];
+  for (int k = 0; k < NP; ++k) a.Mo[k * R + r] = mo[k];
+  a.big[r] = static_cast<unsigned char>(big);
 }
 
 // one degree N of one row from the moments in registers (mo: the row's own,
@@ -297,6 +294,8 @@ __global__ void __launch_bounds__(128) limit_kernel(LimArgs a) {
   using T = typename K::T;
   constexpr int M = K::M, NP = K::NP, P = K::ORDER, NS = K::NS;
   constexpr int NL = P * (P + 1) / 2;  // moments of degrees 0..p-1
+  pdl_trigger();
+  pdl_wait();
   if (a.ctl && a.gctl->done) return;
   const size_t R = (size_t)a.E * M;
   const size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -315,13 +314,13 @@ __global__ void __launch_bounds__(128) limit_kernel(LimArgs a) {
     const int nb[4] = {n4.x, n4.y, n4.z, n4.w};
     double mo[NP], mn[4][NL], rc[4];
 #pragma unroll
-    for (int k = 0; k < NP; ++k) mo[k] = a.Mo[r * NP + k];
+    for (int k = 0; k < NP; ++k) mo[k] = a.Mo[k * R + r];
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
       const int n = nb[d] >= 0 ? nb[d] : e;  // a missing neighbour is never read
-      const double* src = a.Mo + ((size_t)n * M + j) * NP;
+      const double* src = a.Mo + (size_t)n * M + j;
 #pragma unroll
-      for (int k = 0; k < NL; ++k) mn[d][k] = src[k];
+      for (int k = 0; k < NL; ++k) mn[d][k] = src[k * R];
       const double pc = __ldg(a.geo + (size_t)n * kLimGeo + (d < 2 ? 8 : 9));
       const double own = gg[d < 2 ? 4 : 5];
       // left / bottom: own - theirs; right / top: theirs - own
@@ -348,12 +347,13 @@ __global__ void __launch_bounds__(128) limit_kernel(LimArgs a) {
           }
       const T* phif = static_cast<const T*>(a.phif);
       T* tr = static_cast<T*>(a.tr);
-      for (int s = 0; s < NS; ++s) {
-        T acc = 0;
+      if (tr)
+        for (int s = 0; s < NS; ++s) {
+          T acc = 0;
 #pragma unroll
-        for (int k = 0; k < NP; ++k) acc += __ldg(phif + s * NP + k) * ck[k];
-        tr[slot_index<K>(e, s, j)] = acc;
-      }
+          for (int k = 0; k < NP; ++k) acc += __ldg(phif + s * NP + k) * ck[k];
+          tr[slot_index<K>(e, s, j)] = acc;
+        }
     }
   }
   a.trig[r] = static_cast<unsigned char>(trig);

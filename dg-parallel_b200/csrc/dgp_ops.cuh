@@ -22,6 +22,26 @@ constexpr bool adjoint_built() {
 
 constexpr size_t kSmemPerCta = 227 * 1024;
 
+// a launch that may start before the previous kernel of the stream has ended
+// (programmatic dependent launch): the kernel waits itself (pdl_wait) before it
+// touches what earlier kernels write.  Hides the launch and the constant loads:
+// a 20-step run of 2048 P2 triangles 497 -> 430 us, 24 steps of 17554 P1
+// triangles 788 -> 724 us (398 and 703 with the finalize in one round trip).
+template <class... P, class... A>
+void launch_overlapped(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <class K, bool ENS>
 cudaError_t fused_prepare();
 
@@ -143,26 +163,6 @@ size_t ops_fused_smem(int nf_max, int nh_max) {
   return a > b ? a : b;
 }
 
-// a launch that may start before the previous kernel of the stream has ended
-// (programmatic dependent launch): the kernel waits itself (pdl_wait) before it
-// touches what earlier kernels write.  Hides the launch and the constant loads:
-// a 20-step run of 2048 P2 triangles 497 -> 430 us, 24 steps of 17554 P1
-// triangles 788 -> 724 us (398 and 703 with the finalize in one round trip).
-template <class... P, class... A>
-void launch_overlapped(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid));
-  cfg.blockDim = dim3(static_cast<unsigned>(block));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <class K>
 void ops_fused(const DeviceBuffers& b, const double* in, const double* u0, double* out, double* u0copy, int stage,
                double time_factor, int fuse_cfl, cudaStream_t st) {
@@ -245,8 +245,8 @@ void ops_limit(const DeviceBuffers& b, int check_done, cudaStream_t st) {
     a.E = b.E;
     const long long rows = static_cast<long long>(b.E) * K::M;
     const int grid = static_cast<int>((rows + 127) / 128);
-    limit_moments_kernel<K><<<grid, 128, 0, st>>>(a);
-    limit_kernel<K><<<grid, 128, 0, st>>>(a);
+    launch_overlapped(&limit_moments_kernel<K>, grid, 128, 0, st, a);
+    launch_overlapped(&limit_kernel<K>, grid, 128, 0, st, a);
   }
 }
 
@@ -278,7 +278,7 @@ void ops_cfl(const DeviceBuffers& b, cudaStream_t st) {
   StageArgs<typename K::T> a = make_args<typename K::T>(b);
   // ensembles: one block per instance-pure tile
   const int grid = b.cell_inst ? ops_grid_elem<K>(b.E) : (b.E + 255) / 256;
-  cfl_kernel<K><<<grid, 256, 0, st>>>(a);
+  launch_overlapped(&cfl_kernel<K>, grid, 256, 0, st, a);
 }
 
 template <class K>

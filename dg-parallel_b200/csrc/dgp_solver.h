@@ -81,7 +81,7 @@ struct DeviceBuffers {
   double* lim_slope = nullptr;    // Barth: [E][M] slope factors of the pass (written; read when replayed)
   int lim_replay = 0;             // Barth: 1 applies lim_slope instead of computing the factors
   unsigned char* lbig = nullptr;  // [E * M] degrees with a mode above the limiter's threshold
-  double* lmo = nullptr;          // [E * M][NP] moments of every degree of each row
+  double* lmo = nullptr;          // [NP][E * M] moments of every degree of each row
   int* nb = nullptr;              // [E][4] left, right, bottom, top
   double* lgeo = nullptr;         // [E][10] limiter geometry
   double* limD = nullptr;         // derivative tables per degree

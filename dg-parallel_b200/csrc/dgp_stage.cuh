@@ -352,13 +352,6 @@ __device__ __forceinline__ void st_row(double* p, const double (&v)[N]) {
   }
 }
 
-// programmatic dependent launch: the next kernel of the stream may start its
-// CTAs as these leave room (and read what no kernel of the chain writes);
-// pdl_wait returns when the previous kernels have ended and their writes are
-// visible.  Without the launch attribute both do nothing.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
