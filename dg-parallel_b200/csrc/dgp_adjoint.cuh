@@ -25,7 +25,7 @@
 #pragma once
 
 #include "dgp_dual.cuh"
-#include "dgp_elem.cuh"
+#include "dgp_stage.cuh"
 
 namespace dgp {
 
@@ -56,12 +56,23 @@ constexpr int adj_lanes() {
 template <class K>
 __device__ __forceinline__ void nu_trace(const double* __restrict__ mu, double inv_detj,
                                          const typename K::T* phi, typename K::T* V) {
+  // (the vector of the previous launch: plain loads, not the read-only path)
   using T = typename K::T;
+  constexpr int NP = K::NP;
 #pragma unroll
   for (int j = 0; j < K::M; ++j) {
     T acc = 0;
+    if constexpr (NP % 2 == 0) {
 #pragma unroll
-    for (int k = 0; k < K::NP; ++k) acc += phi[k] * (T)__ldg(mu + j * K::NP + k);
+      for (int k = 0; k < NP; k += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(mu + j * NP + k);
+        acc += phi[k] * (T)v.x;
+        acc += phi[k + 1] * (T)v.y;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < NP; ++k) acc += phi[k] * (T)mu[j * NP + k];
+    }
     V[j] = acc * (T)inv_detj;
   }
 }
@@ -77,6 +88,8 @@ __global__ void __launch_bounds__(K::FACE_BLOCK) adj_face_kernel(const __grid_co
   const int tid = threadIdx.x;
   const int fl = tid / NQF, q = tid - (tid / NQF) * NQF;
   const int f = blockIdx.x * K::FPB + fl;
+  pdl_wait();  // (tables and weights are constant; a trigger after the wait keeps the
+  pdl_trigger();  //  stage states that cell_trace reads complete before the kernel starts)
   if (fl >= K::FPB || f >= a.s.mesh.F) return;
   const auto& m = a.s.mesh;
   const int eL = m.fel[2 * f], eR = m.fel[2 * f + 1];
@@ -159,15 +172,14 @@ __global__ void __launch_bounds__(K::FACE_BLOCK) adj_face_kernel(const __grid_co
   for (int c = 0; c < M; ++c) sl[c] = gL[c];
 }
 
+// shared memory of the element kernel: values at the volume points (then
+// U^bar) and H, field-major rows as in the stage kernel
 template <class K>
 struct AdjSmem {
   using T = typename K::T;
-  using L = ElemSmem<K>;
-  static constexpr int NQP = K::NQ | 1;  // row stride of U^bar (odd)
-  static constexpr size_t oU = L::r16(L::bytes);                                   // T [ROWS][NQP]
-  static constexpr size_t oN = oU + L::r16((size_t)K::ROWS * NQP * sizeof(T));     // T [ROWS][NP] nu
-  static constexpr size_t oM = oN + L::r16((size_t)K::ROWS * K::NP * sizeof(T));   // FP64 [ROWS][NP] mu
-  static constexpr size_t bytes = oM + (size_t)K::ROWS * K::NP * 8;
+  using S = StageShape<K>;
+  static constexpr size_t oH = (size_t)S::VQ * S::LDR * sizeof(T);
+  static constexpr size_t bytes = oH + (size_t)S::KV * S::LDR * sizeof(T) + 16;
 };
 
 template <class K>
@@ -175,126 +187,144 @@ constexpr size_t adj_elem_smem() {
   return AdjSmem<K>::bytes;
 }
 
+// Element part of a reversed stage, the work mapping of the stage kernel: one
+// thread per (cell, field) row contracts the stage state and nu from registers
+// against constant-bank tables (U at the volume points, H), thread (cell,
+// point) the flux cotangents on dual numbers, then the rows again.  Linear
+// laws: the volume points are the modes of degree < p (stage kernel), the
+// transposed table and U^bar's modes directly.  P2 Euler on 32768 cells:
+// 30 -> 13 us a launch (tables and rows read from shared memory before).
 template <class K>
-__global__ void __launch_bounds__(K::BLOCK) adj_elem_kernel(const __grid_constant__ AdjArgs<typename K::T> a) {
+__global__ void __launch_bounds__(K::BLOCK) adj_elem_kernel(const __grid_constant__ AdjArgs<typename K::T> a,
+                                                            const __grid_constant__ StageTab<K> tb) {
   using T = typename K::T;
-  using L = ElemSmem<K>;
-  using A = AdjSmem<K>;
-  constexpr int M = K::M, NP = K::NP, NQ = K::NQ, DIM = K::DIM, TE = K::TE, BLOCK = K::BLOCK;
-  constexpr int MNP = K::MNP, NS = K::NS, KV = K::KV, LDK = K::LDK, ROWS = K::ROWS;
-  constexpr int NPP = L::NPP, DD = L::DD, NQP = A::NQP;
+  using S = StageShape<K>;
+  constexpr int M = K::M, NP = K::NP, DIM = K::DIM, TE = K::TE, BLOCK = K::BLOCK;
+  constexpr int NS = K::NS, ROWS = K::ROWS, VQ = S::VQ, KV = S::KV, LDR = S::LDR, TEP = S::TEP;
+  constexpr int RALIGN = pow2_div(NP * 8) < 16 ? pow2_div(NP * 8) : 16;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  T* sT = reinterpret_cast<T*>(smem_raw);
-  const T* sDphi = sT + L::oDphi;
-  const T* sPhif = sT + L::oPhif;
-  const T* sPhi = sT + L::oPhi;
-  const T* sQw = sT + L::oQw;
-  double* sC = reinterpret_cast<double*>(smem_raw + L::oCB);
-  T* sH = reinterpret_cast<T*>(smem_raw + L::oGB);
-  double* sJ = reinterpret_cast<double*>(smem_raw + L::oJB);
-  T* sUb = reinterpret_cast<T*>(smem_raw + A::oU);
-  T* sNu = reinterpret_cast<T*>(smem_raw + A::oN);
-  double* sMu = reinterpret_cast<double*>(smem_raw + A::oM);
+  T* sU = reinterpret_cast<T*>(smem_raw);
+  T* sH = reinterpret_cast<T*>(smem_raw + AdjSmem<K>::oH);
   const int tid = threadIdx.x;
   const int e0 = blockIdx.x * TE;
-  const int ne = min(TE, a.s.mesh.E - e0);
   const auto& m = a.s.mesh;
-
-  for (int i = tid; i < (int)(L::blob_bytes / sizeof(T)); i += BLOCK) sT[i] = a.s.tab.blob[i];
-  for (int i = tid; i < ne * MNP; i += BLOCK) {
-    sC[i] = a.s.C[(size_t)e0 * MNP + i];
-    sMu[i] = a.mu[(size_t)e0 * MNP + i];
-  }
-  for (int i = tid; i < ne * DD; i += BLOCK) {
-    const int e = i / DD, c = i - (i / DD) * DD;
-    sJ[i] = c < DIM * DIM ? (double)m.jinv[(size_t)(e0 + e) * DIM * DIM + c] : m.detjd[e0 + e];
-  }
-  __syncthreads();
-  for (int i = tid; i < ne * MNP; i += BLOCK) sNu[i] = (T)(sMu[i] / sJ[(i / MNP) * DD + DIM * DIM]);
-  __syncthreads();
-
-  // transposed contraction: H[row][kk] = sum_k dphi[kk][k] nu[row][k]
-  const int row = tid;
-  if (row < ne * M) {
-    T nu[NP];
+  const int ne = min(TE, m.E - e0);
+  const int row = tid, cell = row / M, field = row - cell * M, prow = field * TEP + cell;
+  const bool live = row < ne * M;
+  const size_t gbase = ((size_t)e0 * M + row) * NP;
+  const double det = live ? m.detjd[e0 + cell] : 1.0;
+  // a cell's geometry for its points' threads
+  constexpr int NG = BLOCK / TE;
+  const int ve = tid % TE, vg = tid / TE;
+  const bool vlive = vg < NG && ve < ne;
+  T J[DIM * DIM], vdet = 0;
+  if (vlive) {
 #pragma unroll
-    for (int k = 0; k < NP; ++k) nu[k] = sNu[row * NP + k];
-    for (int kk = 0; kk < KV; ++kk) {
-      T acc = 0;
+    for (int i = 0; i < DIM * DIM; ++i) J[i] = m.jinv[(size_t)(e0 + ve) * DIM * DIM + i];
+    vdet = (T)m.detjd[e0 + ve];
+  }
+  pdl_wait();
+  pdl_trigger();
+
+  if (live) {
+    constexpr int UV = table_unroll(VQ > 0 ? VQ : 1, NP), UK = table_unroll(KV > 0 ? KV : 1, NP);
+    double v[NP];
+    T c[NP];
+    ld_row_pinned<NP, RALIGN>(a.s.C + gbase, v);
 #pragma unroll
-      for (int k = 0; k < NP; ++k) acc += sDphi[kk * NPP + k] * nu[k];
-      sH[row * LDK + kk] = acc;
+    for (int k = 0; k < NP; ++k) c[k] = (T)v[k];
+#pragma unroll UV
+    for (int q = 0; q < VQ; ++q) {
+      if constexpr (S::LINEAR)
+        sU[q * LDR + prow] = c[q];
+      else
+        sU[q * LDR + prow] = table_dot<NP, false, T>(c, tb.phi + q * NP, 0);
     }
+    // H[(direction, point)][row] = sum_k dv[(direction, point)][k] nu[row][k]
+    ld_row_pinned<NP, RALIGN>(a.mu + gbase, v);
+#pragma unroll
+    for (int k = 0; k < NP; ++k) c[k] = (T)(v[k] / det);
+#pragma unroll UK
+    for (int kk = 0; kk < KV; ++kk) sH[kk * LDR + prow] = table_dot<NP, false, T>(c, tb.dv + kk * NP, 0);
   }
   __syncthreads();
 
-  // volume: U^bar_m(q) = sum_ji Fbar_ji dF_ji/dU_m at each quadrature point
-  if (tid < K::EG * NQ) {
-    const int q = tid % NQ, g = tid / NQ;
-    T phi[NP];
-#pragma unroll
-    for (int k = 0; k < NP; ++k) phi[k] = sPhi[q * NPP + k];
-    const T w = sQw[q];
+  // U^bar_m(q) = sum_ji Fbar_ji dF_ji/dU_m at each volume point
+  if (vlive) {
     using D = Dual<T, M>;
-    for (int e = g; e < ne; e += K::EG) {
+#pragma unroll 1
+    for (int q = vg; q < VQ; q += NG) {
       D U[M];
 #pragma unroll
-      for (int j = 0; j < M; ++j) {
-        T acc = 0;
-#pragma unroll
-        for (int k = 0; k < NP; ++k) acc += phi[k] * (T)sC[(e * M + j) * NP + k];
-        U[j] = D::var(acc, j);
-      }
+      for (int j = 0; j < M; ++j) U[j] = D::var(sU[q * LDR + j * TEP + ve], j);
       D F[M][DIM];
       volume_flux<K::LAW, DIM, D>(a.s.law, U, F);
-      const double* Jd = sJ + e * DD;
-      const T jw = (T)Jd[DIM * DIM] * w;
+      T jw = vdet;
+      if constexpr (!S::LINEAR) jw = vdet * tb.qw[q];
       T ub[M];
 #pragma unroll
       for (int c = 0; c < M; ++c) ub[c] = 0;
 #pragma unroll
-      for (int j = 0; j < M; ++j)
+      for (int j = 0; j < M; ++j) {
+        T h[DIM];
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) h[r] = sH[(r * VQ + q) * LDR + j * TEP + ve];
 #pragma unroll
         for (int i = 0; i < DIM; ++i) {
           T fb = 0;
 #pragma unroll
-          for (int r = 0; r < DIM; ++r) fb += sH[(e * M + j) * LDK + q * DIM + r] * (T)Jd[i * DIM + r];
+          for (int r = 0; r < DIM; ++r) fb += h[r] * J[i * DIM + r];
           fb *= jw;
 #pragma unroll
           for (int c = 0; c < M; ++c) ub[c] += fb * F[j][i].d[c];
         }
+      }
 #pragma unroll
-      for (int c = 0; c < M; ++c) sUb[(e * M + c) * NQP + q] = ub[c];
+      for (int c = 0; c < M; ++c) sU[q * LDR + c * TEP + ve] = ub[c];
     }
   }
   __syncthreads();
 
   // w = sum_q phi_k(q) U^bar(q) + lift of the adjoint face slots, then the
   // reversed stage combination in FP64
-  if (row < ne * M) {
+  if (live) {
+    double mu[NP], ac[NP];
+    ld_row_pinned<NP, RALIGN>(a.mu + gbase, mu);
+    const bool use_acc = a.cc != 0.0 || a.cd != 0.0;
+    if (use_acc) ld_row_pinned<NP, RALIGN>(a.acc + gbase, ac);
     T acc[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) acc[k] = 0;
-    for (int q = 0; q < NQ; ++q) {
-      const T ub = sUb[row * NQP + q];
+    constexpr int UV = table_unroll(VQ > 0 ? VQ : 1, NP), UF = table_unroll(NS, NP);
+    if constexpr (S::LINEAR) {
 #pragma unroll
-      for (int k = 0; k < NP; ++k) acc[k] += ub * sPhi[q * NPP + k];
+      for (int q = 0; q < VQ; ++q) acc[q] = sU[q * LDR + prow];
+    } else {
+#pragma unroll UV
+      for (int q = 0; q < VQ; ++q) {
+        const T ub = sU[q * LDR + prow];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) acc[k] += ub * tb.phi[q * NP + k];
+      }
     }
     const T* sl = a.s.slots + (size_t)blockIdx.x * NS * ROWS + row;
+#pragma unroll UF
     for (int s = 0; s < NS; ++s) {
-      const T sv = __ldg(sl + (size_t)s * ROWS);
+      const T sv = sl[(size_t)s * ROWS];
 #pragma unroll
-      for (int k = 0; k < NP; ++k) acc[k] += sv * sPhif[s * NPP + k];
+      for (int k = 0; k < NP; ++k) acc[k] += sv * tb.phif[s * NP + k];
     }
-    const size_t gbase = ((size_t)e0 * M + row) * NP;
+    double o[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
-      const double mu = sMu[row * NP + k];
-      const double w = (double)acc[k];
-      double o = a.ca * mu + a.cb * a.dt * w;
-      if (a.cc != 0.0) o += a.cc * a.acc[gbase + k];
-      a.out[gbase + k] = o;
-      if (a.cd != 0.0 || a.ce != 0.0) a.acc[gbase + k] = (a.cd != 0.0 ? a.cd * a.acc[gbase + k] : 0.0) + a.ce * mu;
+      o[k] = a.ca * mu[k] + a.cb * a.dt * (double)acc[k];
+      if (a.cc != 0.0) o[k] += a.cc * ac[k];
+    }
+    st_row<NP, RALIGN>(a.out + gbase, o);
+    if (a.cd != 0.0 || a.ce != 0.0) {
+#pragma unroll
+      for (int k = 0; k < NP; ++k) o[k] = (a.cd != 0.0 ? a.cd * ac[k] : 0.0) + a.ce * mu[k];
+      st_row<NP, RALIGN>(a.acc + gbase, o);
     }
   }
 }

@@ -270,7 +270,7 @@ static std::vector<int> morton_order(const HostMesh& m) {
 }
 
 // Face records and halo sides of the fused stage kernel's tiles (TileMesh):
-// for tile t, every face with a side among its cells, in face order, and the
+// for tile t, every face with a side among its cells, once, and the
 // neighbours' sides of those faces (periodic partners included), sorted by
 // local face so that the kernel's warps contract one face's table rows.  The
 // fused kernel is built for the solver (fused_ok) when every tile's faces and
@@ -287,7 +287,7 @@ static int build_tiles_dim(dgp_solver s, int Etot, const std::vector<int>& fel, 
   struct Counts {
     int halo[5];
   };
-  std::vector<int> fl, foff(1, 0);
+  std::vector<int> fl, foff(1, 0), stamp(fj.size(), -1);
   std::vector<Counts> counts(ntiles);
   std::vector<int2> count(ntiles);
   fl.reserve(fj.size() + fj.size() / 2);
@@ -299,10 +299,10 @@ static int build_tiles_dim(dgp_solver s, int Etot, const std::vector<int>& fel, 
     for (int e = e0; e < e1; ++e)
       for (int lf = 0; lf < nlf; ++lf) {
         const int k = cface[static_cast<size_t>(e) * nlf + lf];
-        if (k >= 0) fl.push_back(k);
+        if (k < 0 || stamp[k] == t) continue;
+        stamp[k] = t;
+        fl.push_back(k);
       }
-    std::sort(fl.begin() + f0, fl.end());
-    fl.erase(std::unique(fl.begin() + f0, fl.end()), fl.end());
     foff.push_back(static_cast<int>(fl.size()));
     Counts c{};
     int nh = 0;

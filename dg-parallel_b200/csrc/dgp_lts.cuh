@@ -22,7 +22,7 @@
 // step captured in a CUDA graph turns into no-ops past the end.
 #pragma once
 
-#include "dgp_kernels.cuh"
+#include "dgp_stage.cuh"
 
 namespace dgp {
 
@@ -64,20 +64,20 @@ __device__ __forceinline__ int lts_segment(const LtsSegs& S, int blk, int& local
 
 // tile shape of the cell kernels: CPB listed cells per 128-thread CTA (one
 // (cell, field) row per thread at most), their coefficients and the volume
-// kernel's flux rows and tables in at most 40 KB of shared memory
+// kernel's point values, field-major as in the stage kernel, in at most 46 KB
+// of shared memory
 template <class K>
 struct LtsTile {
-  static constexpr int M = K::M, MNP = K::MNP, KV = K::KV;
-  static constexpr int KVP = KV | 1;  // row stride of the flux rows (odd: no bank conflicts)
-  // the volume kernel's tables (phi, grad phi, weights) in shared memory when
-  // they take at most 8 KB
-  static constexpr int TAB = K::NQ * K::NP + KV * K::NP + K::NQ;
-  static constexpr bool STAGE_TAB = TAB * 8 <= 8 * 1024;
-  static constexpr int TAB_SMEM = STAGE_TAB ? TAB : 1;
-  static constexpr int BYTES_PER_CELL = 8 * (MNP + M * KVP);
-  static constexpr int BY_ROWS = 128 / M;
-  static constexpr int BY_SMEM = (40 * 1024 - 8 * TAB_SMEM) / BYTES_PER_CELL;
-  static constexpr int CPB = BY_ROWS < BY_SMEM ? BY_ROWS : (BY_SMEM < 1 ? 1 : BY_SMEM);
+  using S = StageShape<K>;
+  static constexpr int M = K::M, MNP = K::MNP;
+  static constexpr int fit() {
+    int c = 128 / M;
+    while (c > 1 && 8 * (c * MNP + S::KV * M * (c + 4)) > 46 * 1024) --c;
+    return c;
+  }
+  static constexpr int CPB = fit();
+  static constexpr int PITCH = field_pitch(CPB, M, 8);
+  static constexpr int LD = M * PITCH;
   static int grid(int n) { return (n + CPB - 1) / CPB; }
 };
 
@@ -103,61 +103,60 @@ __device__ __forceinline__ void lts_add_rows(const int* s_e, int nc, const doubl
 }
 
 // volume term of the listed cells, r[j][k] += sum_q F_j(U_q) . J^-T grad phi_k
-// |J| w_q: one thread per (cell, quadrature point) evaluates the flux once for
-// all fields into the rows G[(cell, j)][(q, r)]; one thread per (cell, field)
-// row contracts its G row with grad phi
+// |J| w_q, in the stage kernel's work mapping: rows contract from registers
+// against the constant-bank tables, thread (cell, point) the flux (linear laws:
+// the modes of degree < p for points).  P3 Euler, a quarter of 32768 cells:
+// 22 -> 14 us a launch (rows and tables from shared memory before).
 template <class K>
 __global__ void __launch_bounds__(128) lts_vol_kernel(const __grid_constant__ StageArgs<double> a,
+                                                       const __grid_constant__ StageTab<K> tb,
                                                        const int* __restrict__ lists,
                                                        const __grid_constant__ LtsSegs S,
                                                        double* __restrict__ racc) {
-  using S_ = LtsTile<K>;
-  constexpr int M = K::M, NP = K::NP, NQ = K::NQ, DIM = K::DIM, MNP = K::MNP, KV = K::KV;
-  constexpr int CPB = S_::CPB, KVP = S_::KVP;
+  using Sh = StageShape<K>;
+  using Tl = LtsTile<K>;
+  constexpr int M = K::M, NP = K::NP, DIM = K::DIM, MNP = K::MNP, VQ = Sh::VQ, KV = Sh::KV;
+  constexpr int CPB = Tl::CPB, PITCH = Tl::PITCH, LD = Tl::LD;
+  constexpr int RALIGN = pow2_div(NP * 8) < 16 ? pow2_div(NP * 8) : 16;
+  constexpr int UV = table_unroll(VQ > 0 ? VQ : 1, NP), UK = table_unroll(VQ > 0 ? VQ : 1, NP * DIM);
   __shared__ double s_c[CPB * MNP];
-  __shared__ double s_g[CPB * M * KVP];
-  __shared__ double s_tab[S_::TAB_SMEM];
+  __shared__ double s_g[KV > 0 ? KV * LD : 1];
   __shared__ int s_e[CPB];
   if (a.gctl->done) return;
   const int tid = threadIdx.x;
-  const double* phi = a.tab.phi;
-  const double* dphi = a.tab.dphi;
-  const double* qw = a.tab.qw;
-  if constexpr (S_::STAGE_TAB) {
-    for (int x = tid; x < NQ * NP; x += 128) s_tab[x] = a.tab.phi[x];
-    for (int x = tid; x < KV * NP; x += 128) s_tab[NQ * NP + x] = a.tab.dphi[x];
-    for (int x = tid; x < NQ; x += 128) s_tab[NQ * NP + KV * NP + x] = a.tab.qw[x];
-    phi = s_tab;
-    dphi = s_tab + NQ * NP;
-    qw = s_tab + NQ * NP + KV * NP;
-  }
   int blk;
   const int sg = lts_segment(S, blockIdx.x, blk);
   const int nc = lts_tile_cells<CPB>(lists + S.off[sg], S.cnt[sg], blk, s_e);
-#pragma unroll 4
-  for (int x = tid; x < nc * MNP; x += 128) {
-    const int i = x / MNP;
-    s_c[x] = a.C[(size_t)s_e[i] * MNP + (x - i * MNP)];
+  const int row = tid, cell = row / M, field = row - cell * M, prow = field * PITCH + cell;
+  const bool live = row < nc * M;
+  if (live) {
+    double c[NP];
+    ld_row_pinned<NP, RALIGN>(a.C + ((size_t)s_e[cell] * M + field) * NP, c);
+#pragma unroll UV
+    for (int q = 0; q < VQ; ++q) {
+      if constexpr (Sh::LINEAR)
+        s_g[q * LD + prow] = c[q];
+      else
+        s_g[q * LD + prow] = table_dot<NP, false, double>(c, tb.phi + q * NP, 0);
+    }
   }
   __syncthreads();
-  for (int x = tid; x < nc * NQ; x += 128) {
-    const int i = x / NQ, q = x - i * NQ, e = s_e[i];
-    const double* c = s_c + i * MNP;
+  for (int x = tid; x < CPB * VQ; x += 128) {
+    const int q = x / CPB, i = x - q * CPB;
+    if (i >= nc) continue;
+    const int e = s_e[i];
     double U[M];
 #pragma unroll
-    for (int jj = 0; jj < M; ++jj) {
-      double u = 0.0;
-#pragma unroll
-      for (int k = 0; k < NP; ++k) u += phi[q * NP + k] * c[jj * NP + k];
-      U[jj] = u;
-    }
-    if (!is_physical<K::LAW, double>(a.law, U)) flag_nonphysical(a.status, e);
+    for (int j = 0; j < M; ++j) U[j] = s_g[q * LD + j * PITCH + i];
+    if (!surely_physical<K::LAW, double>(a.law, U) && !is_physical<K::LAW, double>(a.law, U))
+      flag_nonphysical(a.status, e);
     double F[M][DIM];
     volume_flux<K::LAW, DIM, double>(a.law, U, F);
     double J[DIM * DIM];
 #pragma unroll
     for (int t = 0; t < DIM * DIM; ++t) J[t] = a.mesh.jinv[(size_t)e * DIM * DIM + t];
-    const double jw = a.mesh.detjd[e] * qw[q];
+    double jw = a.mesh.detjd[e];
+    if constexpr (!Sh::LINEAR) jw *= tb.qw[q];
 #pragma unroll
     for (int j = 0; j < M; ++j)
 #pragma unroll
@@ -165,22 +164,26 @@ __global__ void __launch_bounds__(128) lts_vol_kernel(const __grid_constant__ St
         double g = 0.0;
 #pragma unroll
         for (int t = 0; t < DIM; ++t) g += F[j][t] * J[t * DIM + r];
-        s_g[(i * M + j) * KVP + q * DIM + r] = g * jw;
+        s_g[(r * VQ + q) * LD + j * PITCH + i] = g * jw;
       }
   }
   __syncthreads();
-  for (int row = tid; row < nc * M; row += 128) {
+  if (live) {
     double acc[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) acc[k] = 0.0;
-    const double* g = s_g + row * KVP;
-    for (int kk = 0; kk < KV; ++kk) {
-      const double gv = g[kk];
 #pragma unroll
-      for (int k = 0; k < NP; ++k) acc[k] += gv * dphi[kk * NP + k];
+    for (int r = 0; r < DIM; ++r) {
+#pragma unroll UK
+      for (int q = 0; q < VQ; ++q) {
+        const double gv = s_g[(r * VQ + q) * LD + prow];
+#pragma unroll
+        for (int k = 0; k < NP; ++k)
+          if (k >= Sh::k_first(q)) acc[k] += gv * tb.dv[(r * VQ + q) * NP + k];
+      }
     }
 #pragma unroll
-    for (int k = 0; k < NP; ++k) s_c[row * NP + k] = acc[k];  // row < nc * M: own row only
+    for (int k = 0; k < NP; ++k) s_c[row * NP + k] = acc[k];
   }
   __syncthreads();
   lts_add_rows<MNP>(s_e, nc, s_c, racc);
@@ -260,6 +263,7 @@ __global__ void __launch_bounds__(128) lts_lift_kernel(const __grid_constant__ S
 // writes the row's face-point traces from the new coefficients
 template <class K>
 __global__ void __launch_bounds__(128) lts_update_kernel(const __grid_constant__ StageArgs<double> a,
+                                                          const __grid_constant__ StageTab<K> tb,
                                                           const int* __restrict__ lists,
                                                           const __grid_constant__ LtsSegs S,
                                                           double* __restrict__ c1, double* __restrict__ save,
@@ -359,13 +363,10 @@ __global__ void __launch_bounds__(128) lts_update_kernel(const __grid_constant__
     double o[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) o[k] = s_c[row * NP + k];
-#pragma unroll 4
-    for (int s = 0; s < NS; ++s) {
-      double t = 0.0;
-#pragma unroll
-      for (int k = 0; k < NP; ++k) t += a.tab.phif[s * NP + k] * o[k];
-      a.tr[slot_index<K>(e, s, j)] = t;
-    }
+    constexpr int UF = table_unroll(NS, NP);
+    double* tr = a.tr + slot_index<K>(e, 0, j);
+#pragma unroll UF
+    for (int s = 0; s < NS; ++s) tr[(size_t)s * K::ROWS] = table_dot<NP, false, double>(o, tb.phif + s * NP, 0);
   }
 }
 

@@ -42,6 +42,12 @@ void launch_overlapped(void (*kernel)(P...), int grid, int block, size_t smem, c
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// the solver's parameter tables of the instantiation
+template <class K>
+const StageTab<K>& stage_tab(const DeviceBuffers& b) {
+  return *static_cast<const StageTab<K>*>(b.htab);
+}
+
 template <class K, bool ENS>
 cudaError_t fused_prepare();
 
@@ -172,7 +178,7 @@ void ops_fused(const DeviceBuffers& b, const double* in, const double* u0, doubl
   a.Cout = out;
   a.U0out = u0copy;
   a.tab.blob = static_cast<const typename K::T*>(b.fblob);
-  const auto& tb = *static_cast<const StageTab<K>*>(b.htab);
+  const auto& tb = stage_tab<K>(b);
   const int nf = b.tm.nf_max, nh = b.tm.nh_max;
   const int grid = ops_grid_elem<K>(b.E);
   const size_t smem = FusedSmem<K, false>::bytes(nf, nh);
@@ -268,8 +274,8 @@ void ops_adj_stage(const DeviceBuffers& b, const AdjStage& g, cudaStream_t st) {
     a.t_seg = g.t_seg;
     a.t_factor = g.t_factor;
     const int fgrid = (b.F + K::FPB - 1) / K::FPB;
-    adj_face_kernel<K><<<fgrid, K::FACE_BLOCK, 0, st>>>(a);
-    adj_elem_kernel<K><<<ops_grid_elem<K>(b.E), K::BLOCK, adj_elem_smem<K>(), st>>>(a);
+    launch_overlapped(&adj_face_kernel<K>, fgrid, K::FACE_BLOCK, 0, st, a);
+    launch_overlapped(&adj_elem_kernel<K>, ops_grid_elem<K>(b.E), K::BLOCK, adj_elem_smem<K>(), st, a, stage_tab<K>(b));
   }
 }
 
@@ -327,7 +333,7 @@ void ops_lts_vol(const DeviceBuffers& b, const int* lists, const LtsSegs& segs, 
   const StageArgs<double> a = make_args<double>(b);
   LtsSegs S = segs;
   const int grid = lts_fill_blocks(S, LtsTile<K>::CPB);
-  lts_vol_kernel<K><<<grid, 128, 0, st>>>(a, lists, S, racc);
+  lts_vol_kernel<K><<<grid, 128, 0, st>>>(a, stage_tab<K>(b), lists, S, racc);
 }
 
 template <class K>
@@ -351,7 +357,7 @@ void ops_lts_update(const DeviceBuffers& b, const int* lists, const LtsSegs& seg
   const StageArgs<double> a = make_args<double>(b);
   LtsSegs S = segs;
   const int grid = lts_fill_blocks(S, LtsTile<K>::CPB);
-  lts_update_kernel<K><<<grid, 128, 0, st>>>(a, lists, S, c1, save, racc);
+  lts_update_kernel<K><<<grid, 128, 0, st>>>(a, stage_tab<K>(b), lists, S, c1, save, racc);
 }
 
 template <class K>

@@ -61,6 +61,7 @@
 #include <type_traits>
 
 #include "dgp_elem.cuh"
+#include "dgp_host.h"
 #include "dgp_umma.cuh"
 
 namespace dgp {
