@@ -9,7 +9,8 @@
 //   faces   per face point, the traces of nu on both sides give the flux
 //           cotangent Fbar = (nu_R - nu_L) |J_f| w; the Jacobians dF^/dU_L and
 //           dF^/dU_R come from evaluating the law's numerical (or boundary)
-//           flux on dual numbers; U_L^bar = Fbar dF^/dU_L is written into the
+//           flux on dual numbers (the Roe flux: its own reverse pass,
+//           roe_vjp); U_L^bar = Fbar dF^/dU_L is written into the
 //           left cell's face slot, U_R^bar into the right cell's (no atomics,
 //           the forward slot layout);
 //   volume  H[(cell,j)][(q,r)] = sum_k dphi_(q,r),k nu[j][k] (the transposed
@@ -62,7 +63,8 @@ constexpr bool flux_vjp_built() {
 // gL = fb dF^/dU_L, gR = fb dF^/dU_R of the Roe flux (numerical_flux): the
 // reverse pass of its own steps, ~350 operations where 8-lane dual numbers carry
 // nine times the flux's 250 (P2 Euler, 32768 cells: 49 -> 29 us a launch; the
-// whole gradient 6.92 -> 5.88 ms, 6.06 with one block a SM more or less).  x_ stands for the cotangent of x.
+// whole gradient 6.92 -> 5.88 ms at three blocks a SM, 6.02 at four, 6.06 at two).
+// x_ stands for the cotangent of x.
 template <typename T>
 __device__ __forceinline__ void roe_vjp(T g, const T* n, const T* u0, const T* u1, const T* fb, T* gL, T* gR) {
   const T half = (T)0.5, gm1 = g - (T)1, n0 = n[0], n1 = n[1];

@@ -387,11 +387,9 @@ int dgp_backward(dgp_solver s, const double* dJ_duT, double* dJ_du0);
  * element, order, precision, floor(log2 cells)) that dgp_solver_create and
  * dgp_ensemble_create consult (128 threads when nothing is recorded).  For
  * each shape both stage forms are timed where the fused stage kernel is built
- * (dgp_set_fused), and the faster is recorded with it (without a record, a
- * default measured on B200 decides: fused for the 2D Euler (Roe, LLF), scalar
- * and Maxwell laws at P2-P3, 2D Euler P1 and P1 on tets (scalar: P2); the
- * separate kernels for Burgers, the exact Godunov flux, 2D P4, the 3D Euler law
- * and tets of higher order).  ms_per_step[3] (may be NULL) gets each shape's best time, -1
+ * (dgp_set_fused), and the faster is recorded with it (without a record, the
+ * default measured on B200: fused, except for the 3D Euler law's exact Riemann
+ * solver in FP64).  ms_per_step[3] (may be NULL) gets each shape's best time, -1
  * where not built. */
 int dgp_autotune(dgp_mesh m, dgp_law law, int order, int precision, int limiter, int iters, int* best_block,
                  float* ms_per_step);
