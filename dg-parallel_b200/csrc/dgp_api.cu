@@ -892,13 +892,14 @@ int dgp_solver_info(dgp_solver s, int* nfields, int* nmodes, int* ncells, int* n
   return DGP_OK;
 }
 
-static int set_ctl(dgp_solver s, double t, double dt, double tend, double cfl, int max_steps) {
+static int set_ctl(dgp_solver s, double t, double dt, double tend, double cfl, int max_steps, int graph_steps = 0) {
   TimeCtl c{};
   c.t = t;
   c.dt = dt;
   c.tend = tend;
   c.cfl = cfl;
   c.max_steps = max_steps;
+  c.graph_steps = graph_steps;
   c.lts_shift = s->lts.on ? s->lts.nb - 1 : 0;  // mode-5 step: CFL minimum times 2^(bins-1)
   c.dtmin_bits = 0x7FF0000000000000ull;
   s->h_ctl[0] = c;
@@ -1260,13 +1261,15 @@ int dgp_run(dgp_solver s, double t0, double tend, double cfl, int max_steps, dou
   }
   if (tail && !s->graph1)
     if (int rc = capture(1, &s->graph1)) return rc;
-  if (int rc = set_ctl(s, t0, 0.0, tend, cfl, max_steps)) return rc;
+  if (int rc = set_ctl(s, t0, 0.0, tend, cfl, max_steps, K)) return rc;
   if (int rc = reset_probe_recorders(s)) return rc;
   s->ops.cfl(s->b, s->stream);
   DGP_CUDA(cudaGetLastError());
   // Graphs are queued without a host round trip in between as far as the end
   // of the run cannot lie (a step limit exactly, an end time by the last known
   // step, three quarters of it), at most kAhead of them; then the status is read.
+  // A step that is not positive and finite stops the run on the device at the
+  // end of the graph it appears in (ctl_finalize).
   constexpr int kAhead = 8;
   TimeCtl c{};
   long long queued = 0;  // steps
@@ -1284,9 +1287,8 @@ int dgp_run(dgp_solver s, double t0, double tend, double cfl, int max_steps, dou
     if (ones)
       for (; queued < max_steps; ++queued) DGP_CUDA(cudaGraphLaunch(s->graph1, s->stream));
     if (int rc = read_ctl(s, &c)) return rc;
+    if (c.done == kBadStep) return fail(DGP_ERR_NONPHYSICAL, "time step is not positive and finite");
     if (c.done) break;
-    if (!std::isfinite(c.dt) || !(c.dt > 0))
-      return fail(DGP_ERR_NONPHYSICAL, "time step is not positive and finite");
     queued = c.steps;
   }
   if (t_out) *t_out = c.t;

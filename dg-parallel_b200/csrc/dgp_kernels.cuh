@@ -91,6 +91,8 @@ __device__ __forceinline__ size_t slot_index(int e, int s, int j) {
   return ((size_t)(e / K::TE) * K::NS + s) * K::ROWS + (size_t)(e % K::TE) * K::M + j;
 }
 
+constexpr int kBadStep = 2;  // TimeCtl::done: the next time step is not positive and finite
+
 // time-step control that lives in device memory so that a whole run can be
 // captured in a CUDA graph without host round trips
 struct TimeCtl {
@@ -101,11 +103,12 @@ struct TimeCtl {
   double resid;      // sum (u_new - u_n)^2 of the last step
   int steps;         // steps completed
   int max_steps;     // <= 0: unbounded
-  int done;          // set when tend or max_steps is reached
+  int done;          // set when tend or max_steps is reached, or to kBadStep
   int lts_shift;     // local time stepping: the step is the CFL minimum times 2^lts_shift
   unsigned long long dtmin_bits;  // atomicMin accumulator (positive double bits)
   unsigned int blocks_done;       // completion counter of the reducing kernel
-  unsigned int pad2;
+  int graph_steps;                // steps per graph of a run whose graphs are queued ahead of the
+                                  // host (0: no such run)
   unsigned long long t_mark_ns;   // device clock: run start (whole-launch entry) or
                                   // the moment the instance finished (ensembles)
 };
@@ -579,6 +582,13 @@ __device__ __forceinline__ double ctl_finalize(TimeCtl* c, double dtmin) {
   }
   c->dt = dt;
   c->done = done ? 1 : 0;
+  // a run stops between two graphs (of graph_steps steps, then of one each for
+  // what is left under a step limit) where the next step is not positive and
+  // finite; the graphs that are queued behind do nothing
+  if (c->graph_steps > 0 && !done && c->steps > 0 && !(dt > 0 && dt < __longlong_as_double(0x7FF0000000000000ll))) {
+    const int left = c->max_steps > 0 ? c->max_steps % c->graph_steps : 0;
+    if (c->steps % c->graph_steps == 0 || (left > 0 && c->steps >= c->max_steps - left)) c->done = kBadStep;
+  }
   return dt;
 }
 
