@@ -305,23 +305,23 @@ __global__ void __launch_bounds__(K::BLOCK) adj_elem_kernel(const __grid_constan
                                                             const __grid_constant__ StageTab<K> tb) {
   using T = typename K::T;
   using S = StageShape<K>;
-  constexpr int M = K::M, NP = K::NP, DIM = K::DIM, TE = K::TE, BLOCK = K::BLOCK;
-  constexpr int NS = K::NS, ROWS = K::ROWS, VQ = S::VQ, KV = S::KV, LDR = S::LDR, TEP = S::TEP;
+  constexpr int M = K::M, NP = K::NP, DIM = K::DIM, TS = K::TS, BLOCK = K::BLOCK;
+  constexpr int NS = K::NS, VQ = S::VQ, KV = S::KV, LDR = S::LDR, TEP = S::TEP;
   constexpr int RALIGN = pow2_div(NP * 8) < 16 ? pow2_div(NP * 8) : 16;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   T* sU = reinterpret_cast<T*>(smem_raw);
   T* sH = reinterpret_cast<T*>(smem_raw + AdjSmem<K>::oH);
   const int tid = threadIdx.x;
-  const int e0 = blockIdx.x * TE;
+  const int e0 = blockIdx.x * TS;
   const auto& m = a.s.mesh;
-  const int ne = min(TE, m.E - e0);
+  const int ne = min(TS, m.E - e0);
   const int row = tid, cell = row / M, field = row - cell * M, prow = field * TEP + cell;
   const bool live = row < ne * M;
   const size_t gbase = ((size_t)e0 * M + row) * NP;
   const double det = live ? m.detjd[e0 + cell] : 1.0;
   // a cell's geometry for its points' threads
-  constexpr int NG = BLOCK / TE;
-  const int ve = tid % TE, vg = tid / TE;
+  constexpr int NG = BLOCK / TS;
+  const int ve = tid % TS, vg = tid / TS;
   const bool vlive = vg < NG && ve < ne;
   T J[DIM * DIM], vdet = 0;
   if (vlive) {
@@ -413,10 +413,10 @@ __global__ void __launch_bounds__(K::BLOCK) adj_elem_kernel(const __grid_constan
         for (int k = 0; k < NP; ++k) acc[k] += ub * tb.phi[q * NP + k];
       }
     }
-    const T* sl = a.s.slots + (size_t)blockIdx.x * NS * ROWS + row;
+    const T* sl = a.s.slots + slot_index<K>(e0 + cell, 0, field);
 #pragma unroll UF
     for (int s = 0; s < NS; ++s) {
-      const T sv = sl[(size_t)s * ROWS];
+      const T sv = sl[(size_t)s * K::ROWS];
 #pragma unroll
       for (int k = 0; k < NP; ++k) acc[k] += sv * tb.phif[s * NP + k];
     }

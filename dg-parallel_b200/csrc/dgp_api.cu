@@ -272,16 +272,13 @@ static std::vector<int> morton_order(const HostMesh& m) {
 // Face records and halo sides of the fused stage kernel's tiles (TileMesh):
 // for tile t, every face with a side among its cells, once, and the
 // neighbours' sides of those faces (periodic partners included), sorted by
-// local face so that the kernel's warps contract one face's table rows.  The
-// fused kernel is built for the solver (fused_ok) when every tile's faces and
-// halo fit in shared memory; whether the stages then use it or the face and
-// element kernels is tuned_fused's choice (dgp_set_fused switches).
+// local face so that the kernel's warps contract one face's table rows.
 template <int DIM>
 static int build_tiles_dim(dgp_solver s, int Etot, const std::vector<int>& fel, const std::vector<int>& fcode,
                            const std::vector<double>& fnrm, const std::vector<double>& fj,
                            const std::vector<int>& bpart, const std::vector<int>& cface) {
-  const int TE = s->ops.TE, nlf = s->tab.nlf;
-  const int ntiles = (Etot + TE - 1) / TE;
+  const int TS = s->ops.TS, nlf = s->tab.nlf;
+  const int ntiles = (Etot + TS - 1) / TS;
   // the tiles' faces and their halo sides' counts by local face (4: periodic
   // partners)
   struct Counts {
@@ -294,7 +291,7 @@ static int build_tiles_dim(dgp_solver s, int Etot, const std::vector<int>& fel, 
   foff.reserve(ntiles + 1);
   int nh_max = 1, nf_max = 1;
   for (int t = 0; t < ntiles; ++t) {
-    const int e0 = t * TE, e1 = std::min(e0 + TE, Etot);
+    const int e0 = t * TS, e1 = std::min(e0 + TS, Etot);
     const size_t f0 = fl.size();
     for (int e = e0; e < e1; ++e)
       for (int lf = 0; lf < nlf; ++lf) {
@@ -318,16 +315,10 @@ static int build_tiles_dim(dgp_solver s, int Etot, const std::vector<int>& fel, 
     nh_max = std::max(nh_max, nh);
     nf_max = std::max(nf_max, nf);
   }
-  s->fused_ok = s->ops.fused != nullptr && nlf * TE <= kHaloRef && bpart.size() < (1u << 26) &&
-                s->ops.fused_smem(nf_max, nh_max) + 4 * 1024 <= 227 * 1024;
-  long long cells = 0;
-  for (const auto& hm : s->meshes) cells += hm.E;
-  s->fused = s->fused_ok && tuned_fused(s->law, s->flux, DIM, s->order, s->precision, cells);
-  if (!s->fused_ok) return DGP_OK;
   std::vector<FaceRec<DIM>> rec(static_cast<size_t>(ntiles) * nf_max);
   std::vector<int2> th_side(static_cast<size_t>(ntiles) * nh_max, make_int2(-1, 0));
   for (int t = 0; t < ntiles; ++t) {
-    const int e0 = t * TE, e1 = std::min(e0 + TE, Etot);
+    const int e0 = t * TS, e1 = std::min(e0 + TS, Etot);
     auto own = [&](int e) { return e >= e0 && e < e1; };
     int place[5], nh = 0;
     for (int c = 0; c < 5; ++c) {
@@ -345,10 +336,10 @@ static int build_tiles_dim(dgp_solver s, int Etot, const std::vector<int>& fel, 
       const int eL = fel[2 * static_cast<size_t>(k)], eR = fel[2 * static_cast<size_t>(k) + 1];
       const int lfL = fcode[k] & 15, lfR = (fcode[k] >> 4) & 15, perm = (fcode[k] >> 8) & 15;
       FaceRec<DIM> r{};
-      unsigned side = own(eL) ? lfL * TE + (eL - e0) : halo(eL, lfL, lfL);
+      unsigned side = own(eL) ? lfL * TS + (eL - e0) : halo(eL, lfL, lfL);
       int kind = kFaceInterior, bnd = 0;
       if (eR >= 0) {
-        side |= static_cast<unsigned>(own(eR) ? lfR * TE + (eR - e0) : halo(eR, lfR, lfR)) << 16;
+        side |= static_cast<unsigned>(own(eR) ? lfR * TS + (eR - e0) : halo(eR, lfR, lfR)) << 16;
       } else {
         bnd = -eR - 1;
         kind = kFaceBoundary;
@@ -387,13 +378,26 @@ static int build_tiles(dgp_solver s, int Etot, const std::vector<int>& fel, cons
 
 // Builds the device state of a solver over the instances already in s->meshes
 // (one mesh for a single solver).  Instance i owns internal cells
-// [inst_off[i], inst_off[i] + E_i), each instance starting on an
-// element-kernel tile; ensemble=false keeps the single-solver layout (no
-// per-instance arrays, kernels see cell_inst == nullptr).
-static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int field, bool ensemble) {
+// [inst_off[i], inst_off[i] + E_i), each instance starting on a tile of the
+// stage form; ensemble=false keeps the single-solver layout (no per-instance
+// arrays, kernels see cell_inst == nullptr).  The fused stage kernel is built
+// (fused_ok) for every mesh whose boundary faces its records can number; form:
+// 1 / 0 the stages through it or through the face and element kernels, -1
+// tuned_fused's choice (dgp_set_fused switches a single solver).
+static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int field, bool ensemble, int form = -1) {
   const int n = static_cast<int>(s->meshes.size());
   const int dim = s->meshes[0].dim;
   const int TE = s->ops.TE;
+  long long cells = 0, nbound = 0;
+  for (const auto& hm : s->meshes) {
+    cells += hm.E;
+    nbound += std::count_if(hm.eR.begin(), hm.eR.end(), [](int e) { return e < 0; });
+  }
+  s->fused_ok = s->ops.fused != nullptr && nbound < (1LL << 26);
+  s->fused = s->fused_ok && (form < 0 ? tuned_fused(s->law, s->flux, dim, s->order, s->precision, cells) : form == 1);
+  // an ensemble's instances start on the tiles of its form, which it keeps
+  const int tile = s->fused ? s->ops.TS : TE;
+  if (ensemble) s->fused_ok = s->fused;
   const RefTables& t = s->tab;
   s->inst_off.resize(n);
   s->inst_ufirst.resize(n);
@@ -403,7 +407,7 @@ static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int fie
     s->inst_ufirst[i] = uf;
     const int Ei = s->meshes[i].E;
     uf += Ei;
-    Etot += ensemble ? (Ei + TE - 1) / TE * TE : Ei;
+    Etot += ensemble ? (Ei + tile - 1) / tile * tile : Ei;
     Ftot += s->meshes[i].F;
   }
   DeviceBuffers& b = s->b;
@@ -532,7 +536,8 @@ static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int fie
   }
   b.F = Ftot;
   b.NB = nb;
-  if (int rc = build_tiles(s, Etot, fel, fcode, fnrm, fj, bpart, cface)) return rc;
+  if (s->fused_ok)
+    if (int rc = build_tiles(s, Etot, fel, fcode, fnrm, fj, bpart, cface)) return rc;
   // per-cell geometry padded to whole tiles (the element kernel copies a
   // tile's J^{-1} and |J| in one piece)
   {
@@ -636,13 +641,14 @@ static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int fie
     std::vector<int> inst_end(n), tile_first(n + 1);
     for (int i = 0; i < n; ++i) {
       inst_end[i] = s->inst_off[i] + s->meshes[i].E;
-      tile_first[i] = s->inst_off[i] / TE;
+      tile_first[i] = s->inst_off[i] / tile;
     }
-    tile_first[n] = (Etot + TE - 1) / TE;
+    tile_first[n] = Etot / tile;
     if ((rc = s->upload(&b.cell_inst, cell_inst)) || (rc = s->upload(&b.inst_end, inst_end)) ||
         (rc = s->upload(&b.tile_first, tile_first)) || (rc = s->upload(&b.laws, lps)))
       return rc;
     b.ninst = n;
+    b.ens_tile = tile;
   }
   Status st0{0, INT32_MAX};
   DGP_CUDA(cudaMemcpy(b.status, &st0, sizeof(Status), cudaMemcpyHostToDevice));
@@ -1532,8 +1538,9 @@ int dgp_synchronize(dgp_solver s) {
 // clock).  Groups run on their own streams; a run is a loop of CUDA-graph
 // launches of 8 steps per group until every instance is done.
 
-int dgp_ensemble_create(int n, const dgp_mesh* meshes, const dgp_law* laws, const int* orders, int precision,
-                        int limiter, dgp_ensemble* out) {
+// form: the groups' stage form (build_solver)
+static int ensemble_create(int n, const dgp_mesh* meshes, const dgp_law* laws, const int* orders, int precision,
+                           int limiter, int form, dgp_ensemble* out) {
   if (n <= 0 || !meshes || !laws || !orders || !out) return fail(DGP_ERR_INVALID, "bad argument");
   if (precision != DGP_PRECISION_FP64 && precision != DGP_PRECISION_MIXED)
     return fail(DGP_ERR_INVALID, "unknown precision");
@@ -1583,7 +1590,7 @@ int dgp_ensemble_create(int n, const dgp_mesh* meshes, const dgp_law* laws, cons
       e->inst_group[i] = static_cast<int>(e->groups.size());
       e->inst_index[i] = static_cast<int>(k);
     }
-    if (int rc = build_solver(s, lps, l0->field, true)) {
+    if (int rc = build_solver(s, lps, l0->field, true, form)) {
       delete s;
       delete e;
       return rc;
@@ -1593,6 +1600,11 @@ int dgp_ensemble_create(int n, const dgp_mesh* meshes, const dgp_law* laws, cons
   e->n = n;
   *out = e;
   return DGP_OK;
+}
+
+int dgp_ensemble_create(int n, const dgp_mesh* meshes, const dgp_law* laws, const int* orders, int precision,
+                        int limiter, dgp_ensemble* out) {
+  return ensemble_create(n, meshes, laws, orders, precision, limiter, -1, out);
 }
 
 int dgp_ensemble_destroy(dgp_ensemble e) {
@@ -1942,24 +1954,24 @@ int dgp_autotune_ensemble(int n, const dgp_mesh* meshes, const dgp_law* laws, co
     for (int block : kTileBlocks) {
       if (!has_block(law, flux, dim, order, precision, block)) continue;
       set_tuned_block(law, flux, dim, order, precision, cells, block);
-      dgp_ensemble e = nullptr;
-      if (int rc = dgp_ensemble_create(static_cast<int>(ms.size()), ms.data(), ls.data(), os.data(), precision,
-                                       limiter, &e))
-        return rc;
-      dgp_solver g = e->groups[0];
-      int rc = DGP_OK;
-      for (int f = 0; f < (g->fused_ok ? 2 : 1) && !rc; ++f) {
-        if (g->fused_ok) rc = dgp_set_fused(g, f);
+      for (int f = 0; f < 2; ++f) {  // both stage forms, each with its own layout
+        dgp_ensemble e = nullptr;
+        if (int rc = ensemble_create(static_cast<int>(ms.size()), ms.data(), ls.data(), os.data(), precision,
+                                     limiter, f, &e))
+          return rc;
+        dgp_solver g = e->groups[0];
+        const bool fused = g->fused;
         float t = 0;
-        if (!rc) rc = time_steps(g, iters, &t);
-        if (!rc && (!best || t < best_ms)) {
+        int rc = DGP_OK;
+        if (fused == (f == 1)) rc = time_steps(g, iters, &t);
+        dgp_ensemble_destroy(e);
+        if (rc) return rc;
+        if (fused == (f == 1) && (!best || t < best_ms)) {
           best = block;
           best_ms = t;
-          best_fused = g->fused_ok && f == 1;
+          best_fused = fused;
         }
       }
-      dgp_ensemble_destroy(e);
-      if (rc) return rc;
     }
     if (best) {
       set_tuned_block(law, flux, dim, order, precision, cells, best);
@@ -1979,7 +1991,7 @@ int dgp_tune_set(int law, int flux, int dim, int order, int precision, int cells
 int dgp_solver_block(dgp_solver s, int* block, int* cells_per_tile) {
   if (!s) return fail(DGP_ERR_INVALID, "null solver");
   if (block) *block = s->ops.elem_block;
-  if (cells_per_tile) *cells_per_tile = s->ops.TE;
+  if (cells_per_tile) *cells_per_tile = s->fused ? s->ops.TS : s->ops.TE;
   return DGP_OK;
 }
 
@@ -1992,7 +2004,7 @@ int dgp_solver_fused(dgp_solver s, int* fused) {
 int dgp_set_fused(dgp_solver s, int on) {
   if (!s) return fail(DGP_ERR_INVALID, "null solver");
   if (on && !s->fused_ok)
-    return fail(DGP_ERR_UNSUPPORTED, "no fused stage kernel for this solver (a tile's halo does not fit)");
+    return fail(DGP_ERR_UNSUPPORTED, "no fused stage kernel for this solver");
   if (on == (s->fused ? 1 : 0)) return DGP_OK;
   DGP_CUDA(cudaSetDevice(s->device));
   s->drop_graphs();

@@ -67,13 +67,23 @@ struct Cfg {
   // geometry, CFL eigenvalues
   static constexpr int CELL_BYTES = 16 * MNP + (int)sizeof(T) * (M * LDK + NS * M) + 8 * (NV + DIM * DIM + 1);
   // shared-memory budget of a tile of the element kernel: 768 bytes per
-  // thread, at most 96 KB so that two tiles (with the table blob) share an SM;
-  // up to P2 on tets and P4 on triangles every row thread then has a row
-  static constexpr int SMEM_BUDGET = BLOCK * 768 < 96 * 1024 ? BLOCK * 768 : 96 * 1024;
+  // thread, at most 64 KB so that three tiles (with the table blob) share an SM
+  // whatever the order
+  static constexpr int SMEM_BUDGET = BLOCK * 768 < 64 * 1024 ? BLOCK * 768 : 64 * 1024;
   static constexpr int TE_SMEM = SMEM_BUDGET / CELL_BYTES;
   static constexpr int TE_ROWS = BLOCK / M;
   static constexpr int TE = TE_SMEM < TE_ROWS ? (TE_SMEM < 1 ? 1 : TE_SMEM) : TE_ROWS;
   static constexpr int ROWS = TE * M;
+  // cells per tile of the fused stage kernel (and the adjoint's element
+  // kernel), which keep less of a cell in shared memory: up to P2 on tets and
+  // P4 on triangles every row thread has a row.  The element kernel loses at
+  // this size where it leaves one tile fewer on an SM (FP64, a step, its own
+  // tile / this one: Maxwell P2 tets 696 / 739 us, P3 2315 / 2639, scalar P3
+  // tets 534 / 597, 3D Euler P3 2794 / 3076, Euler P4 844 / 878; 93750 tets,
+  // 131072 triangles).
+  static constexpr int STAGE_BUDGET = BLOCK * 768 < 96 * 1024 ? BLOCK * 768 : 96 * 1024;
+  static constexpr int TS_SMEM = STAGE_BUDGET / CELL_BYTES;
+  static constexpr int TS = TS_SMEM < TE_ROWS ? (TS_SMEM < 1 ? 1 : TS_SMEM) : TE_ROWS;
   static constexpr int EG = BLOCK / NQ;   // cells processed concurrently in the volume phase
   // face slots live tile-transposed, [tile][face point][row], so that the
   // element kernel reads them row-coalesced: slot(e, s, j) =
@@ -164,7 +174,7 @@ struct DevTables {
 };
 
 // One face of a tile in the fused stage kernel (read whole from shared
-// memory).  A side is an own side, (local face) * TE + local cell, or with
+// memory).  A side is an own side, (local face) * TS + local cell, or with
 // kHaloRef set the index of a halo side of the tile.
 constexpr int kHaloRef = 0x8000;
 constexpr int kFaceInterior = 0, kFaceBoundary = 1, kFacePeriodic = 2;
@@ -177,7 +187,7 @@ struct alignas(16) FaceRec {
 };
 
 // Per-tile face records and halo sides of the fused stage kernel.  Tile t
-// owns cells [t TE, (t + 1) TE); its faces are every face with a side in the
+// owns cells [t TS, (t + 1) TS); its faces are every face with a side in the
 // tile (a face between two tiles appears in both lists and is evaluated by
 // both, identically).  A halo side is a neighbour's side of such a face, or a
 // periodic partner; sides are sorted by local face.
@@ -219,7 +229,8 @@ struct StageArgs {
   TimeCtl* gctl;
   const int* cell_inst;    // [E] instance of each cell (-1: padding)
   const int* inst_end;     // [ninst] one past the last cell of each instance
-  const int* tile_first;   // [ninst + 1] first element-kernel tile of each instance
+  const int* tile_first;   // [ninst + 1] first tile of each instance
+  int ens_tile;            // cells per tile of an ensemble: the tiles of its stage form
   const LawParams* laws;   // [ninst] field parameters of each instance
   int ninst;
   int stage;       // 0: RHS only, 1..3: SSP-RK3 stages
@@ -660,8 +671,8 @@ __device__ __forceinline__ void finalize_instances(const StageArgs<T>& a, bool a
 }
 
 // CFL reduction of the first step (and, with the limiter, after the last
-// stage's limiter pass).  Ensembles reduce per instance over instance-pure
-// tiles of TE cells, one tile per block.
+// stage's limiter pass).  Ensembles reduce per instance over the instance-pure
+// tiles of their stage form, one tile per block.
 template <class K>
 __global__ void __launch_bounds__(256) cfl_kernel(const __grid_constant__ StageArgs<typename K::T> a) {
   __shared__ double red[256 / 32];
@@ -673,12 +684,12 @@ __global__ void __launch_bounds__(256) cfl_kernel(const __grid_constant__ StageA
   int e = blockIdx.x * 256 + threadIdx.x, eend = a.mesh.E;
   bool active = true;
   if (a.cell_inst) {
-    const int e0 = blockIdx.x * K::TE;
+    const int e0 = blockIdx.x * a.ens_tile;
     const int inst = a.cell_inst[e0];
     c = a.ctl + inst;
     active = !c->done;
-    e = threadIdx.x < K::TE ? e0 + threadIdx.x : a.mesh.E;
-    eend = min(e0 + K::TE, a.inst_end[inst]);
+    e = threadIdx.x < a.ens_tile ? e0 + threadIdx.x : a.mesh.E;
+    eend = min(e0 + a.ens_tile, a.inst_end[inst]);
   }
   double dtl = 1e300;
   if (active && e < eend) dtl = cell_dt<K>(a, a.C + (size_t)e * K::MNP, e, c->cfl);

@@ -104,6 +104,11 @@ int ops_grid_elem(int E) {
 }
 
 template <class K>
+int ops_grid_stage(int E) {
+  return (E + K::TS - 1) / K::TS;
+}
+
+template <class K>
 StageArgs<typename K::T> stage_args(const DeviceBuffers& b, int stage, double time_factor, int fuse_cfl) {
   using T = typename K::T;
   StageArgs<T> a = make_args<T>(b);
@@ -163,15 +168,18 @@ void ops_stage(const DeviceBuffers& b, int stage, double time_factor, int fuse_c
   ops_elem<K>(b, stage, fuse_cfl, st);
 }
 
-template <class K>
-size_t ops_fused_smem(int nf_max, int nh_max) {
-  const size_t a = FusedSmem<K, false>::bytes(nf_max, nh_max), b = FusedSmem<K, true>::bytes(nf_max, nh_max);
-  return a > b ? a : b;
+// every face of every cell of a tile its own record and a halo side
+template <class K, bool TC>
+constexpr size_t fused_smem_worst() {
+  return FusedSmem<K, TC>::bytes(K::NLF * K::TS, K::NLF * K::TS);
 }
 
 template <class K>
 void ops_fused(const DeviceBuffers& b, const double* in, const double* u0, double* out, double* u0copy, int stage,
                double time_factor, int fuse_cfl, cudaStream_t st) {
+  static_assert(K::NLF * K::TS <= kHaloRef && fused_smem_worst<K, false>() <= kSmemPerCta - 4096 &&
+                    fused_smem_worst<K, true>() <= kSmemPerCta - 4096,
+                "a tile of any mesh fits in shared memory");
   auto a = stage_args<K>(b, stage, time_factor, fuse_cfl);
   a.C = in;
   a.U0 = u0;
@@ -180,7 +188,7 @@ void ops_fused(const DeviceBuffers& b, const double* in, const double* u0, doubl
   a.tab.blob = static_cast<const typename K::T*>(b.fblob);
   const auto& tb = stage_tab<K>(b);
   const int nf = b.tm.nf_max, nh = b.tm.nh_max;
-  const int grid = ops_grid_elem<K>(b.E);
+  const int grid = ops_grid_stage<K>(b.E);
   const size_t smem = FusedSmem<K, false>::bytes(nf, nh);
   auto kernel = b.cell_inst ? &stage_kernel<K, true, false> : &stage_kernel<K, false, false>;
   size_t bytes = smem;
@@ -275,7 +283,7 @@ void ops_adj_stage(const DeviceBuffers& b, const AdjStage& g, cudaStream_t st) {
     a.t_factor = g.t_factor;
     const int fgrid = (b.F + K::FPB - 1) / K::FPB;
     launch_overlapped(&adj_face_kernel<K>, fgrid, K::FACE_BLOCK, 0, st, a);
-    launch_overlapped(&adj_elem_kernel<K>, ops_grid_elem<K>(b.E), K::BLOCK, adj_elem_smem<K>(), st, a, stage_tab<K>(b));
+    launch_overlapped(&adj_elem_kernel<K>, ops_grid_stage<K>(b.E), K::BLOCK, adj_elem_smem<K>(), st, a, stage_tab<K>(b));
   }
 }
 
@@ -283,7 +291,7 @@ template <class K>
 void ops_cfl(const DeviceBuffers& b, cudaStream_t st) {
   StageArgs<typename K::T> a = make_args<typename K::T>(b);
   // ensembles: one block per instance-pure tile
-  const int grid = b.cell_inst ? ops_grid_elem<K>(b.E) : (b.E + 255) / 256;
+  const int grid = b.cell_inst ? (b.E + b.ens_tile - 1) / b.ens_tile : (b.E + 255) / 256;
   launch_overlapped(&cfl_kernel<K>, grid, 256, 0, st, a);
 }
 
@@ -368,6 +376,7 @@ Ops make_ops() {
   o.NQ = K::NQ;
   o.NQF = K::NQF;
   o.TE = K::TE;
+  o.TS = K::TS;
   o.elem_block = K::BLOCK;
   o.fpb = K::FPB;
   o.elem_smem = elem_kernel_smem<K>();
@@ -386,7 +395,6 @@ Ops make_ops() {
   o.face = &ops_face<K>;
   o.elem = &ops_elem<K>;
   o.fused = &ops_fused<K>;
-  o.fused_smem = &ops_fused_smem<K>;
   o.cfl = &ops_cfl<K>;
   o.project = &ops_project<K>;
   o.l2err = &ops_l2err<K>;

@@ -93,6 +93,7 @@ struct DeviceBuffers {
   int* tile_first = nullptr;
   LawParams* laws = nullptr;
   int ninst = 0;
+  int ens_tile = 0;  // cells per tile of an ensemble (its instances start on tiles)
 };
 
 template <typename T>
@@ -153,6 +154,7 @@ inline StageArgs<T> make_args(const DeviceBuffers& b) {
   a.tile_first = b.tile_first;
   a.laws = b.laws;
   a.ninst = b.ninst;
+  a.ens_tile = b.ens_tile;
   a.order = b.order;
   return a;
 }
@@ -172,7 +174,7 @@ struct AdjStage {
 
 // Kernel set of one instantiation.
 struct Ops {
-  int M = 0, NP = 0, NQ = 0, NQF = 0, TE = 0, elem_block = 0, precision = 0;
+  int M = 0, NP = 0, NQ = 0, NQF = 0, TE = 0, TS = 0, elem_block = 0, precision = 0;
   int fpb = 0;  // faces per face-kernel CTA
   size_t elem_smem = 0;
   size_t tsize = 8;
@@ -199,7 +201,6 @@ struct Ops {
   // the input rows in stage 1
   void (*fused)(const DeviceBuffers&, const double* in, const double* u0, double* out, double* u0copy, int stage,
                 double time_factor, int fuse_cfl, cudaStream_t) = nullptr;
-  size_t (*fused_smem)(int nf_max, int nh_max) = nullptr;
   void (*cfl)(const DeviceBuffers&, cudaStream_t) = nullptr;
   void (*project)(const DeviceBuffers&, double t, cudaStream_t) = nullptr;
   // over cells [e_begin, e_end); lp: field parameters (nullptr: the solver's law)

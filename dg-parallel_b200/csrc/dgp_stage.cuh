@@ -1,4 +1,4 @@
-// Fused stage kernel: one CTA per tile of TE cells computes every face flux
+// Fused stage kernel: one CTA per tile of TS cells computes every face flux
 // that touches the tile, the volume term, the lift of the face slots, the
 // diagonal inverse mass and the SSP-RK3 stage combination, with the last
 // stage's residual and CFL reductions fused in.
@@ -121,7 +121,7 @@ struct StageShape {
   // volume points: quadrature points, or the modes of degree < p
   static constexpr int VQ = LINEAR ? modes_upto(K::DIM, K::ORDER - 1) : K::NQ;
   static constexpr int KV = VQ * K::DIM;
-  static constexpr int TEP = field_pitch(K::TE, K::M, sizeof(T));
+  static constexpr int TEP = field_pitch(K::TS, K::M, sizeof(T));
   // pitch of a face or volume point: the points of a face (consecutive lanes
   // of phase B) fall on banks apart
   static constexpr int LANES = 128 / (int)sizeof(T);
@@ -199,7 +199,7 @@ struct FusedSmem {
   // with split operands) where TC asks for it: one M = 128 MMA tile covers
   // the tile's rows, N = 16 the modes, K = KPAD the (direction, point) pairs
   // padded to whole k-steps.  UMMA_OK: the shape allows it.
-  static constexpr bool UMMA_OK = MIXED && K::BLOCK == 128 && K::ROWS <= 128 && K::NP <= 16;
+  static constexpr bool UMMA_OK = MIXED && K::BLOCK == 128 && K::TS * K::M <= 128 && K::NP <= 16;
   static constexpr bool UMMA = UMMA_OK && TC;
   static constexpr int KPAD = S::KV > 0 ? (S::KV + 7) / 8 * 8 : 8;
   static constexpr int UN = 16;
@@ -210,7 +210,7 @@ struct FusedSmem {
   static constexpr size_t fblob_elems = UMMA_OK ? 2 * b_bytes / 4 : 1;
   // one-field laws keep the volume values in registers
   static constexpr bool VREG = K::M == 1 && !UMMA;
-  static constexpr size_t rows_bytes = (size_t)K::TE * K::MNP * 8;
+  static constexpr size_t rows_bytes = (size_t)K::TS * K::MNP * 8;
   static constexpr bool bulk_rows = rows_bytes % 16 == 0;  // every tile starts on a 16-byte boundary
   static constexpr size_t max2(size_t a, size_t b) { return a > b ? a : b; }
   // slots (later the CFL states, FP64) | volume values (r = 0 of G) |
@@ -223,8 +223,8 @@ struct FusedSmem {
   static constexpr size_t oJ =
       oX + r16(max2(r16(rows_bytes), UMMA ? 2 * a_bytes
                                           : VREG ? 0 : (size_t)(K::DIM - 1) * S::VQ * S::LDR * sizeof(T)));
-  static constexpr size_t oDet = oJ + r16((size_t)K::TE * K::DIM * K::DIM * sizeof(T));
-  static constexpr size_t oB = oDet + r16((size_t)K::TE * 8);
+  static constexpr size_t oDet = oJ + r16((size_t)K::TS * K::DIM * K::DIM * sizeof(T));
+  static constexpr size_t oB = oDet + r16((size_t)K::TS * 8);
   static constexpr size_t oF = oB + (UMMA ? r16(2 * b_bytes) : 0);
   static constexpr bool P0 = has_physical_range(K::LAW);
   static constexpr size_t halo_bytes = (size_t)S::LDH * sizeof(T) + (P0 ? (size_t)K::M * 2 * sizeof(T) : 0);
@@ -235,7 +235,7 @@ struct FusedSmem {
   __host__ __device__ static constexpr size_t oM(int nf, int nh) {
     return oP(nf, nh) + (P0 ? r16((size_t)nh * K::M * 2 * sizeof(T)) : 0);
   }
-  static constexpr size_t bytes(int nf, int nh) { return oM(nf, nh) + (P0 ? r16((size_t)K::TE + nh) : 0); }
+  static constexpr size_t bytes(int nf, int nh) { return oM(nf, nh) + (P0 ? r16((size_t)K::TS + nh) : 0); }
   // at most 128 registers a thread (FP32: 80), so that four (six) CTAs of 128
   // threads fit; P3 Euler Roe on 131072 cells, a stage: FP64 89 us at 128 and
   // 89 at 168 (three CTAs), FP32 58 at 80, 61 at 100, 67 at 128
@@ -365,7 +365,7 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
 template <class K>
 __device__ __forceinline__ void fused_tile_idle(const StageArgs<typename K::T>& a, int tile) {
   if (a.stage != 3 || threadIdx.x != 0) return;
-  const int ntiles = (a.mesh.E + K::TE - 1) / K::TE;
+  const int ntiles = (a.mesh.E + K::TS - 1) / K::TS;
   a.partials[tile] = 0.0;
   a.partials[ntiles + tile] = 1e300;
 }
@@ -395,7 +395,7 @@ __device__ __forceinline__ bool fused_face_point(const StageArgs<typename K::T>&
                                                  unsigned char* s_mark, bool check) {
   using T = typename K::T;
   using S = StageShape<K>;
-  constexpr int M = K::M, NQF = K::NQF, DIM = K::DIM, TE = K::TE;
+  constexpr int M = K::M, NQF = K::NQF, DIM = K::DIM, TS = K::TS;
   const int refL = fr.side & 0xffff, refR = (unsigned)fr.side >> 16;
   const int kind = (fr.code >> 3) & 3;
   T n[DIM];
@@ -404,7 +404,7 @@ __device__ __forceinline__ bool fused_face_point(const StageArgs<typename K::T>&
   const T jw = probe<RND, T>((T)fr.fj * s_fqw[q], a.round_mask, kRndGeometry);
   // an own side's trace lies in the slots, a halo side's in its own list
   const bool ownL = !(refL & kHaloRef);
-  const int lfL = refL / TE, lL = refL - lfL * TE;
+  const int lfL = refL / TS, lL = refL - lfL * TS;
   T* pL = sS + (lfL * NQF + q) * S::LDR + lL;
   bool marked = false;
   T UL[M], UR[M], flux[M];
@@ -430,8 +430,8 @@ __device__ __forceinline__ bool fused_face_point(const StageArgs<typename K::T>&
         qR = s_qmap[perm * NQF + q];
     }
     if (ownR) {
-      const int lfR = refR / TE;
-      lR = refR - lfR * TE;
+      const int lfR = refR / TS;
+      lR = refR - lfR * TS;
       pR = sS + (lfR * NQF + qR) * S::LDR + lR;
 #pragma unroll
       for (int j = 0; j < M; ++j) UR[j] = pR[j * S::TEP];
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
   using S = StageShape<K>;
   using FS = FusedSmem<K, TC>;
   constexpr int M = K::M, NP = K::NP, MNP = K::MNP, NS = K::NS, NQF = K::NQF, DIM = K::DIM;
-  constexpr int TE = K::TE, NT = K::BLOCK, VQ = S::VQ, KV = S::KV, LDR = S::LDR, TEP = S::TEP, NV = K::NV;
+  constexpr int TS = K::TS, NT = K::BLOCK, VQ = S::VQ, KV = S::KV, LDR = S::LDR, TEP = S::TEP, NV = K::NV;
   constexpr bool PHYS = has_physical_range(K::LAW);
   constexpr int RALIGN = pow2_div(NP * 8) < 16 ? pow2_div(NP * 8) : 16;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
 
   const int tid = threadIdx.x;
   const int tile = blockIdx.x;
-  const int e0 = tile * TE;
+  const int e0 = tile * TS;
   const int nfm = a.tm.nf_max, nhm = a.tm.nh_max;
   T* sHt = reinterpret_cast<T*>(smem_raw + FS::oH(nfm));
   T* sBnd = reinterpret_cast<T*>(smem_raw + FS::oP(nfm, nhm));
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
   // a stored state of an odd length), B of the tensor cores.  A bound on the
   // first wait (a.mbar_polls) counts polls from the rows' issue.
   pdl_trigger();
-  const int nrow = min(TE, a.mesh.E - e0);
+  const int nrow = min(TS, a.mesh.E - e0);
   const bool bulk = FS::bulk_rows && (nrow * MNP) % 2 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
   const uint32_t rb = bulk ? (uint32_t)(nrow * MNP * 8) : 0u;
   bool failed = false;
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
     csz = ld_pinned(a.mesh.csize + e0 + tid);
   if (tid < NQF) s_fqw[tid] = tb.fqw[tid];
   if constexpr (PHYS)
-    for (int i = tid; i < TE + nhm; i += NT) s_mark[i] = 0;
+    for (int i = tid; i < TS + nhm; i += NT) s_mark[i] = 0;
   int inst = 0, eend = a.mesh.E;
   if constexpr (ENS) {  // the tile belongs to one instance
     inst = a.cell_inst[e0];
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
     }
     return;
   }
-  const int ne = min(TE, eend - e0), nf = cnt.x, nh = cnt.y;
+  const int ne = min(TS, eend - e0), nf = cnt.x, nh = cnt.y;
 
   const int row = tid;
   const bool live = row < ne * M;
@@ -655,8 +655,8 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
   const int prow = field * TEP + cell;
   const size_t gbase = ((size_t)e0 * M + row) * NP;
   // volume point owner (laws with several fields): cell ve, points vg, vg + NG, ...
-  constexpr int NG = NT / TE;
-  const int ve = tid % TE, vg = tid / TE;
+  constexpr int NG = NT / TS;
+  const int ve = tid % TS, vg = tid / TS;
   T accv[FS::VREG ? NP : 1];  // volume term of a one-field law's row
 
   // a second round only when the P0 fallback dropped a cell of the tile
@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
       for (int k = 0; k < NP; ++k) hc[k] = (T)hrow[k];
       if constexpr (PHYS) {
         if (round > 0) {
-          if (s_mark[TE + h])
+          if (s_mark[TS + h])
 #pragma unroll
             for (int k = 1; k < NP; ++k) hc[k] = (T)0;
         } else if (a.p0) {
@@ -771,7 +771,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
       if (a.p0 && round == 0) {
         for (int h = tid; h < nh; h += NT)
           if (halo_cell_bad<K>(a, tb, a.tm.th_side + (size_t)tile * nhm + h, sBnd + 2 * h * M)) {
-            s_mark[TE + h] = 1;
+            s_mark[TS + h] = 1;
             mk = true;
           }
       }
@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
   // its cells (DGCell::computeMAXEV, DGCell.cc:1155-1207: eigenvalue at the
   // mean and, on triangles, at the three reference vertices), written to
   // partials[tile] and partials[ntiles + tile] for stage_finalize_kernel
-  const int ntiles = (a.mesh.E + TE - 1) / TE;
+  const int ntiles = (a.mesh.E + TS - 1) / TS;
   double dtl = 1e300;
   if (a.fuse_cfl) {
     if constexpr (state_dependent_speed(K::LAW)) {
@@ -1024,7 +1024,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
         }
       }
       __syncthreads();
-      for (int i0 = 0; i0 < TE * NV; i0 += NT) {
+      for (int i0 = 0; i0 < TS * NV; i0 += NT) {
         const int e = (i0 + tid) / NV, v = (i0 + tid) % NV;
         double am = 0.0;
         if (e < ne) {

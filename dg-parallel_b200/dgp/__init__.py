@@ -408,7 +408,7 @@ class Solver:
         return bins, role
 
     def block(self) -> tuple[int, int]:
-        """(threads, cells per element-kernel tile) of the tile shape in use."""
+        """(threads, cells per tile) of the stage form in use."""
         b, te = ctypes.c_int(), ctypes.c_int()
         check(lib().dgp_solver_block(self.h, ctypes.byref(b), ctypes.byref(te)))
         return b.value, te.value
@@ -616,7 +616,7 @@ class Ensemble:
         return n.value
 
     def group_block(self, g: int) -> tuple[int, int]:
-        """(threads, cells per element-kernel tile) of kernel group g."""
+        """(threads, cells per tile) of kernel group g."""
         b, te = ctypes.c_int(), ctypes.c_int()
         check(lib().dgp_ensemble_group_block(self.h, g, ctypes.byref(b), ctypes.byref(te)))
         return b.value, te.value

@@ -398,6 +398,7 @@ int dgp_autotune_ensemble(int n, const dgp_mesh* meshes, const dgp_law* laws, co
                           int limiter, int iters);
 /* records a tile shape by hand (as the autotuner would) for meshes of `cells` cells */
 int dgp_tune_set(int law, int flux, int dim, int order, int precision, int cells, int block);
+/* the tile shape: threads, and cells per tile of the stage form in use */
 int dgp_solver_block(dgp_solver s, int* block, int* cells_per_tile);
 int dgp_ensemble_group_block(dgp_ensemble e, int group, int* block, int* cells_per_tile);
 #ifdef __cplusplus
