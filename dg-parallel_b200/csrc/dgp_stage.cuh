@@ -784,7 +784,10 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
 #pragma unroll
         for (int i = 0; i < DIM * DIM; ++i) J[i] = sJi[row * DIM * DIM + i];
         const T det = (T)sDet[row];
-        constexpr int UV = table_unroll(VQ > 0 ? VQ : 1, NP * (1 + DIM));
+        // linear laws whole: the entries that vanish are then known when the
+        // kernel is compiled (P3 tets, 381 of 600: left in a loop, their test
+        // cost 1124 us a step of 93750 cells in FP64 against 466, 728 / 251 mixed)
+        constexpr int UV = S::LINEAR ? (VQ > 0 ? VQ : 1) : table_unroll(VQ > 0 ? VQ : 1, NP * (1 + DIM));
 #pragma unroll UV
         for (int q = 0; q < VQ; ++q) {
           T U[1], F[1][DIM];
