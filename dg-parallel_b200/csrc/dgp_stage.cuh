@@ -238,8 +238,12 @@ struct FusedSmem {
   static constexpr size_t bytes(int nf, int nh) { return oM(nf, nh) + (P0 ? r16((size_t)K::TS + nh) : 0); }
   // at most 128 registers a thread (FP32: 80), so that four (six) CTAs of 128
   // threads fit; P3 Euler Roe on 131072 cells, a stage: FP64 89 us at 128 and
-  // 89 at 168 (three CTAs), FP32 58 at 80, 61 at 100, 67 at 128
-  static constexpr int REGS = MIXED ? 80 : 128;
+  // 89 at 168 (three CTAs), FP32 58 at 80, 61 at 100, 67 at 128.  FP32 takes 128
+  // where 80 cost more in spills than the CTAs gain: rows of 15 modes and more
+  // (P4 triangles, P3 tets), and the tensor-core form whose A operand leaves no
+  // room for more than four CTAs (P3 and P4).
+  static constexpr int SMEM_CTAS = (int)(227 * 1024 / (bytes(2 * K::TS, K::TS) + 1024));
+  static constexpr int REGS = MIXED && K::NP < 15 && !(UMMA && SMEM_CTAS <= 4) ? 80 : 128;
   static constexpr int MIN_BLOCKS = 65536 / (K::BLOCK * REGS) > 0 ? 65536 / (K::BLOCK * REGS) : 1;
 };
 
@@ -545,7 +549,7 @@ __device__ __forceinline__ void own_points(const StageTab<K>& tb, const typename
 }
 
 template <class K, bool ENS, bool TC = false, bool RND = false>
-__global__ void __launch_bounds__(K::BLOCK, FusedSmem<K>::MIN_BLOCKS)
+__global__ void __launch_bounds__(K::BLOCK, FusedSmem<K, TC>::MIN_BLOCKS)
     stage_kernel(const __grid_constant__ StageArgs<typename K::T> a, const __grid_constant__ StageTab<K> tb) {
   using T = typename K::T;
   using S = StageShape<K>;
