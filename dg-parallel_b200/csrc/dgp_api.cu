@@ -82,22 +82,42 @@ void set_tuned_block(int law, int flux, int dim, int order, int precision, long 
 // there is one, else the default below.
 std::map<std::tuple<int, int, int, int, int, int>, int> g_tune_fused;
 
-// Step times on B200, separate over fused, 100k-180k cells: 1.3-2.6 everywhere
-// on triangles (1.06-1.25 with the exact Riemann solver, FP64), 1.8-2.1 on tets
-// -- but 0.6-0.7 for the exact Riemann solver on tets in FP64, whose faces
-// between two tiles (every third) the fused form evaluates twice at ~700
-// operations a point (mixed: 1.00-1.07).
-bool fused_default(int law, int flux, int dim, int order, int precision) {
-  (void)flux;
-  (void)dim;
-  (void)order;
-  return !(law == DGP_LAW_EULER3D && precision == DGP_PRECISION_FP64);
+// Step times on B200, separate over fused (800 to 524288 cells):
+//   triangles P0-P3 and P4 of the linear laws 1.1-3.1; P4 of the others
+//     (0.64, 0.90 for Burgers) at 3200 cells, 1.0-1.2 at 8192, 1.1-2.0 above,
+//     the exact Riemann solver's in FP64 (0.90) at 8192, 1.05 at 32768: a few
+//     tiles expose the fetch of a stage's unrolled code;
+//   P0 of the Euler laws, which leaves the point work a face between two tiles
+//     costs twice: FP64 triangles 1.8-2.0 up to 16200 cells, 1.13 at 65522,
+//     (0.90) at 131072, the exact Riemann solver's 0.95 and (0.76), tets 1.6 at
+//     7986, (0.98) at 24576; mixed 1.0 or more but for the exact Riemann solver,
+//     (0.98) at 131072, on tets 1.05 at 48000, (0.88) at 93750;
+//   tets P1 1.8-2.1, P2 0.9 at 8000, 1.4-2.7 above; P3, 20 modes a row, of the
+//     scalar law (0.67) at 7986, 1.2-1.9 above, of Maxwell's in FP64 (0.6-1.0
+//     but for 1.27 at 24576), mixed (0.81) at 3072, 1.4-1.7 above;
+//   the exact Riemann solver on tets (P1-P3): FP64 (0.5-0.7), for about half of
+//     the faces lie between two tiles and are solved twice at ~700 operations a
+//     point; mixed P1 1.0-1.1, (0.92) at 384000, P2 (0.9) at 3072, 1.0-1.3
+//     above, (0.89) at 384000, P3 (0.6-0.9).
+// Brackets: the separate kernels are the default.
+bool fused_default(int law, int flux, int dim, int order, int precision, long long cells) {
+  const bool fp64 = precision == DGP_PRECISION_FP64, riemann = flux == DGP_FLUX_GODUNOV;
+  const bool euler = law == DGP_LAW_EULER2D || law == DGP_LAW_EULER3D;
+  if (euler && order == 0) {
+    if (dim == 3) return cells < (fp64 ? 20000 : 60000);
+    return fp64 ? cells < 80000 : !riemann || cells < 120000;
+  }
+  if (dim == 2) return order < 4 || !(euler || law == DGP_LAW_BURGERS2D) || cells >= (riemann && fp64 ? 24000 : 6000);
+  if (law == DGP_LAW_EULER3D)
+    return !fp64 && (order == 1 || (order == 2 && cells >= 6000)) && cells < 200000;
+  if (order < 3) return true;
+  return law == DGP_LAW_SCALAR ? cells >= 16000 : !fp64 && cells >= 5000;
 }
 
 bool tuned_fused(int law, int flux, int dim, int order, int precision, long long cells) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto it = g_tune_fused.find(std::make_tuple(law, flux, dim, order, precision, size_bucket(cells)));
-  return it == g_tune_fused.end() ? fused_default(law, flux, dim, order, precision) : it->second != 0;
+  return it == g_tune_fused.end() ? fused_default(law, flux, dim, order, precision, cells) : it->second != 0;
 }
 
 void set_tuned_fused(int law, int flux, int dim, int order, int precision, long long cells, bool fused) {

@@ -6,7 +6,7 @@ import pytest
 
 import dgp
 from dgp import meshgen
-from cases import PULSE3D, SINE, TM110, VORTEX, rel
+from cases import PULSE3D, SCALAR2D, SCALAR3D, SINE, TM110, VORTEX, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -36,6 +36,23 @@ def test_forms_have_their_own_tiles(kind, order, elem, stage):
     s.set_state(u0)
     assert s.run(0.0, 0.0, 0.1, 3)[1] == n == 3
     assert rel(s.get_state(), u) < 1e-12
+
+
+# the default form at sizes where the other one was measured slower or faster
+@pytest.mark.parametrize("kind,order,precision,n,fused", [
+    ("scalar3d", 3, dgp.FP64, 4, False), ("scalar3d", 3, dgp.MIXED, 15, True), ("scalar3d", 2, dgp.FP64, 4, True),
+    ("maxwell3d", 3, dgp.FP64, 4, False), ("maxwell3d", 3, dgp.MIXED, 4, False), ("maxwell3d", 3, dgp.MIXED, 10, True),
+    ("euler3d", 1, dgp.FP64, 4, False), ("euler3d", 1, dgp.MIXED, 4, True), ("euler3d", 3, dgp.MIXED, 10, False),
+    ("euler", 4, dgp.FP64, 20, False), ("euler", 4, dgp.FP64, 60, True), ("euler", 3, dgp.FP64, 20, True),
+    ("euler", 0, dgp.FP64, 20, True), ("euler", 0, dgp.FP64, 210, False), ("scalar", 4, dgp.FP64, 20, True)])
+def test_default_form(kind, order, precision, n, fused):
+    args = {"scalar3d": (dgp.LAW_SCALAR, dgp.FLUX_UPWIND, dgp.FIELD_GAUSS3D, SCALAR3D),
+            "scalar": (dgp.LAW_SCALAR, dgp.FLUX_UPWIND, dgp.FIELD_GAUSS, SCALAR2D),
+            "maxwell3d": (dgp.LAW_MAXWELL3D, dgp.FLUX_UPWIND, dgp.FIELD_TM110, TM110),
+            "euler3d": (dgp.LAW_EULER3D, dgp.FLUX_GODUNOV, dgp.FIELD_PULSE3D, PULSE3D),
+            "euler": (dgp.LAW_EULER2D, dgp.FLUX_ROE, dgp.FIELD_VORTEX, VORTEX)}[kind]
+    s = dgp.Solver(_mesh(3 if kind.endswith("3d") else 2, n, 3, box=10.0), dgp.Law(*args), order, precision)
+    assert s.fused == fused
 
 
 # an ensemble of each form whose tiles differ (17 / 25 cells, 14 / 21), in FP64
