@@ -230,13 +230,13 @@ struct StageArgs {
   const int* cell_inst;    // [E] instance of each cell (-1: padding)
   const int* inst_end;     // [ninst] one past the last cell of each instance
   const int* tile_first;   // [ninst + 1] first tile of each instance
-  int ens_tile;            // cells per tile of an ensemble: the tiles of its stage form
   const LawParams* laws;   // [ninst] field parameters of each instance
   int ninst;
   int stage;       // 0: RHS only, 1..3: SSP-RK3 stages
   int fuse_cfl;    // stage 3 reduces the next step's dt
   int order;
   int p0;          // 1: P0 fallback on (face kernel marks, element kernel consumes marks)
+  int ens_tile;    // ensembles: cells per tile of the stage form
 };
 
 // programmatic dependent launch: the next kernel of the stream may start its

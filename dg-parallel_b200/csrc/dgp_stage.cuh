@@ -138,9 +138,10 @@ struct StageShape {
   }
 };
 
-// The reference tables as the kernel's parameters.
+// The reference tables as the kernel's parameters, on 16 bytes whatever comes
+// before them: the wide constant loads of neighbouring entries need it.
 template <class K>
-struct StageTab {
+struct alignas(16) StageTab {
   using T = typename K::T;
   using S = StageShape<K>;
   T phif[K::NS * K::NP];                       // face traces [local face, point][mode]
