@@ -82,24 +82,26 @@ void set_tuned_block(int law, int flux, int dim, int order, int precision, long 
 // there is one, else the default below.
 std::map<std::tuple<int, int, int, int, int, int>, int> g_tune_fused;
 
-// Step times on B200, separate over fused (800 to 524288 cells):
-//   triangles P0-P3 and P4 of the linear laws 1.1-3.1; P4 of the others
-//     (0.64, 0.90 for Burgers) at 3200 cells, 1.0-1.2 at 8192, 1.1-2.0 above,
-//     the exact Riemann solver's in FP64 (0.90) at 8192, 1.05 at 32768: a few
-//     tiles expose the fetch of a stage's unrolled code;
+// Step times on B200, separate over fused (800 to 524288 triangles, 750 to
+// 384000 tets; brackets: the separate kernels are the default):
+//   triangles P0-P3, and P4 of the linear laws, 1.1-3.1;
+//   P4 of the others in FP64 (0.64, Burgers 0.96) at 3200 cells, 1.0-1.1 at
+//     8192, 1.1-2.0 above; mixed (0.99) at 800, 1.0-1.2 at 3200, 1.2-2.0 above;
+//     the exact Riemann solver in FP64 (0.95) at 16200, 1.06 at 32768, mixed
+//     (0.93) at 3200, 1.09 at 8192: a few tiles expose the fetch of a stage's
+//     unrolled code;
 //   P0 of the Euler laws, which leaves the point work a face between two tiles
-//     costs twice: FP64 triangles 1.8-2.0 up to 16200 cells, 1.13 at 65522,
-//     (0.90) at 131072, the exact Riemann solver's 0.95 and (0.76), tets 1.6 at
+//     costs twice: FP64 triangles 1.8-1.9 up to 16200 cells, 1.13 at 65522,
+//     (0.89) at 131072, the exact Riemann solver 0.95 and (0.75), tets 1.6 at
 //     7986, (0.98) at 24576; mixed 1.0 or more but for the exact Riemann solver,
-//     (0.98) at 131072, on tets 1.05 at 48000, (0.88) at 93750;
-//   tets P1 1.8-2.1, P2 0.9 at 8000, 1.4-2.7 above; P3, 20 modes a row, of the
-//     scalar law (0.67) at 7986, 1.2-1.9 above, of Maxwell's in FP64 (0.6-1.0
-//     but for 1.27 at 24576), mixed (0.81) at 3072, 1.4-1.7 above;
-//   the exact Riemann solver on tets (P1-P3): FP64 (0.5-0.7), for about half of
-//     the faces lie between two tiles and are solved twice at ~700 operations a
-//     point; mixed P1 1.0-1.1, (0.92) at 384000, P2 (0.9) at 3072, 1.0-1.3
-//     above, (0.89) at 384000, P3 (0.6-0.9).
-// Brackets: the separate kernels are the default.
+//     (0.98) at 131072, on tets 1.04 at 48000, (0.89) at 93750;
+//   tets P0, P1 1.1-2.1, P2 0.9 at 8000, 1.4-2.7 above; P3, 20 modes a row, of
+//     the scalar law (0.67) at 7986, 1.1-1.9 above, of Maxwell's in FP64
+//     (0.6-1.0 but for 1.27 at 24576), mixed (0.81) at 3072, 1.5-1.6 above;
+//   the exact Riemann solver on tets: FP64 (0.5-0.8), for about half of the
+//     faces lie between two tiles and are solved twice at ~700 operations a
+//     point; mixed P1 1.0-1.1, (0.98) at 196608, P2 (0.96) at 7986, 1.25 at
+//     24576, 1.06 at 48000, (0.95) at 93750, P3 (0.6-0.95).
 bool fused_default(int law, int flux, int dim, int order, int precision, long long cells) {
   const bool fp64 = precision == DGP_PRECISION_FP64, riemann = flux == DGP_FLUX_GODUNOV;
   const bool euler = law == DGP_LAW_EULER2D || law == DGP_LAW_EULER3D;
@@ -107,9 +109,14 @@ bool fused_default(int law, int flux, int dim, int order, int precision, long lo
     if (dim == 3) return cells < (fp64 ? 20000 : 60000);
     return fp64 ? cells < 80000 : !riemann || cells < 120000;
   }
-  if (dim == 2) return order < 4 || !(euler || law == DGP_LAW_BURGERS2D) || cells >= (riemann && fp64 ? 24000 : 6000);
-  if (law == DGP_LAW_EULER3D)
-    return !fp64 && (order == 1 || (order == 2 && cells >= 6000)) && cells < 200000;
+  if (dim == 2) {
+    if (order < 4 || !(euler || law == DGP_LAW_BURGERS2D)) return true;
+    return cells >= (riemann ? (fp64 ? 24000 : 6000) : (fp64 ? 6000 : 2000));
+  }
+  if (law == DGP_LAW_EULER3D) {
+    if (fp64 || order > 2) return false;
+    return order == 1 ? cells < 150000 : cells >= 12000 && cells < 70000;
+  }
   if (order < 3) return true;
   return law == DGP_LAW_SCALAR ? cells >= 16000 : !fp64 && cells >= 5000;
 }
