@@ -124,9 +124,8 @@ struct dgp_solver_s {
   int* d_i2f = nullptr;
   int* d_f2i = nullptr;
   std::vector<void*> allocs;
-  cudaGraphExec_t graph = nullptr;   // graph_steps SSP-RK3 steps
+  cudaGraphExec_t graph = nullptr;   // kGraphSteps steps
   cudaGraphExec_t graph1 = nullptr;  // one step (the tail of a run with a step limit)
-  int graph_steps = 0;
   dgp::TimeCtl* h_ctl = nullptr;  // pinned, 2 entries
   LtsState lts;                    // local time stepping (off unless enabled)
   std::vector<double> stage_tab;   // host storage of b.htab
