@@ -62,6 +62,7 @@
 
 #include "dgp_elem.cuh"
 #include "dgp_host.h"
+#include "dgp_round.h"
 #include "dgp_umma.cuh"
 
 namespace dgp {
@@ -318,15 +319,6 @@ __device__ __forceinline__ int2 ld_pinned_i2(const int2* p) {
   int2 v;
   asm volatile("ld.global.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
-}
-
-// x / 3, rounded correctly: the product with the reciprocal, corrected by its
-// exact remainder (Markstein 1990); infinities pass through the product
-__device__ __forceinline__ double third(double x) {
-  const double y = 1.0 / 3.0;
-  const double q = x * y;
-  const double r = __fma_rn(-3.0, q, x);
-  return r == r ? __fma_rn(r, y, q) : q;
 }
 
 // a row of N FP64 values at p, aligned to ALIGN bytes
