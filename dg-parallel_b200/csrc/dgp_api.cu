@@ -602,7 +602,6 @@ static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int fie
     std::vector<double> phimax(np, 0.0);
     for (size_t i = 0; i < t.phi.size(); ++i) phimax[i % np] = std::max(phimax[i % np], std::fabs(t.phi[i]));
     for (size_t i = 0; i < t.phif.size(); ++i) phimax[i % np] = std::max(phimax[i % np], std::fabs(t.phif[i]));
-    if ((rc = s->upload_t(&b.phimax, phimax))) return rc;
     s->stage_tab.resize(s->ops.stage_tab_bytes / 8 + 1);
     s->ops.fill_stage_tab(t, phimax.data(), s->stage_tab.data());
     b.htab = s->stage_tab.data();

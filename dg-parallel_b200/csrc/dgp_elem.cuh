@@ -355,8 +355,7 @@ struct GeoArea {
   static constexpr size_t oJi = oEig + 8 * (size_t)K::TE * K::NV;
 };
 
-// One CTA per tile of TE cells.  Used where the persistent kernel's 16-byte
-// alignment conditions do not hold.
+// One CTA per tile of TE cells.
 template <class K>
 __global__ void __launch_bounds__(K::BLOCK) elem_kernel(const __grid_constant__ StageArgs<typename K::T> a) {
   using T = typename K::T;

@@ -68,7 +68,7 @@ struct Cfg {
   static constexpr int CELL_BYTES = 16 * MNP + (int)sizeof(T) * (M * LDK + NS * M) + 8 * (NV + DIM * DIM + 1);
   // shared-memory budget of a tile of the element kernel: 768 bytes per
   // thread, at most 64 KB so that three tiles (with the table blob) share an SM
-  // whatever the order
+  // (two at P3 on tets, whose blob takes up to 24 KB)
   static constexpr int SMEM_BUDGET = BLOCK * 768 < 64 * 1024 ? BLOCK * 768 : 64 * 1024;
   static constexpr int TE_SMEM = SMEM_BUDGET / CELL_BYTES;
   static constexpr int TE_ROWS = BLOCK / M;
@@ -93,7 +93,6 @@ struct Cfg {
   // that measured fastest
   static constexpr int FACE_BLOCK = 128;
   static constexpr int FPB = FACE_BLOCK / NQF;  // faces per face-kernel CTA
-  static constexpr int LDM = MNP | 1;           // staged coefficient row stride
 };
 
 template <class K>
@@ -161,7 +160,6 @@ struct DevTables {
   const T* fqw;     // NQF
   const int* qmap;  // NPERM x NQF
   const double* phiv;  // (DIM+1) x NP  (FP64, CFL)
-  const T* phimax;     // NP: largest |phi_k| over the volume and face points (P0 check)
   const double* phiq;  // NQ x NP (FP64, projection)
   const double* qwd;   // NQ (FP64)
   const double* qpd;   // NQ x 3 (FP64)

@@ -229,7 +229,6 @@ struct FusedSmem {
   static constexpr size_t oB = oDet + r16((size_t)K::TS * 8);
   static constexpr size_t oF = oB + (UMMA ? r16(2 * b_bytes) : 0);
   static constexpr bool P0 = has_physical_range(K::LAW);
-  static constexpr size_t halo_bytes = (size_t)S::LDH * sizeof(T) + (P0 ? (size_t)K::M * 2 * sizeof(T) : 0);
   __host__ __device__ static constexpr size_t oH(int nf) { return oF + (size_t)nf * sizeof(FaceRec<K::DIM>); }
   __host__ __device__ static constexpr size_t oP(int nf, int nh) {
     return oH(nf) + r16((size_t)nh * S::LDH * sizeof(T));
