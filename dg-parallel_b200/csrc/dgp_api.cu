@@ -924,14 +924,14 @@ int dgp_solver_info(dgp_solver s, int* nfields, int* nmodes, int* ncells, int* n
   return DGP_OK;
 }
 
-static int set_ctl(dgp_solver s, double t, double dt, double tend, double cfl, int max_steps, int graph_steps = 0) {
+static int set_ctl(dgp_solver s, double t, double dt, double tend, double cfl, int max_steps, int one_from = 0) {
   TimeCtl c{};
   c.t = t;
   c.dt = dt;
   c.tend = tend;
   c.cfl = cfl;
   c.max_steps = max_steps;
-  c.graph_steps = graph_steps;
+  c.one_from = one_from;
   c.lts_shift = s->lts.on ? s->lts.nb - 1 : 0;  // mode-5 step: CFL minimum times 2^(bins-1)
   c.dtmin_bits = 0x7FF0000000000000ull;
   s->h_ctl[0] = c;
@@ -1263,12 +1263,10 @@ int dgp_step(dgp_solver s, double t, double dt, double* resid) {
   return DGP_OK;
 }
 
-// steps per graph of a run
-constexpr int kGraphSteps = 8;
-
-// A graph of `steps` steps of the solver, captured where a run first needs it
-// (a local step is ~90 launches: a run of two that also captured the graph of
-// eight took 3.6 ms where it takes 2.4, and 1.6 the next time).
+// A graph of `steps` steps of the solver, captured once: the one that a run
+// starts with before its first launch, the other while the device is busy with
+// the first (a local step is ~90 launches, and capturing eight of them takes
+// what the device takes for one).
 static int step_graph(dgp_solver s, int steps, cudaGraphExec_t* out) {
   if (*out) return DGP_OK;
   cudaGraph_t g;
@@ -1295,7 +1293,13 @@ int dgp_run(dgp_solver s, double t0, double tend, double cfl, int max_steps, dou
   const int K = kGraphSteps;
   const bool tail = max_steps > 0 && max_steps % K != 0;
   if (s->lts.on) refresh_traces(s);
-  if (int rc = set_ctl(s, t0, 0.0, tend, cfl, max_steps, K)) return rc;
+  if (max_steps > 0 && max_steps < K && tend <= 0) {
+    if (int rc = step_graph(s, 1, &s->graph1)) return rc;
+  } else if (int rc = step_graph(s, K, &s->graph)) {
+    return rc;
+  }
+  if (int rc = set_ctl(s, t0, 0.0, tend, cfl, max_steps, tail ? std::max(max_steps - max_steps % K, 1) : INT32_MAX))
+    return rc;
   if (int rc = reset_probe_recorders(s)) return rc;
   s->ops.cfl(s->b, s->stream);
   DGP_CUDA(cudaGetLastError());
@@ -1316,14 +1320,16 @@ int dgp_run(dgp_solver s, double t0, double tend, double cfl, int max_steps, dou
     int n = static_cast<int>(std::min<long long>(left / K, kAhead));
     const bool ones = tail && left == max_steps - queued && n < kAhead;
     if (n == 0 && !ones) n = 1;
-    if (n > 0)
-      if (int rc = step_graph(s, K, &s->graph)) return rc;
+    for (int i = 0; i < n; ++i) DGP_CUDA(cudaGraphLaunch(s->graph, s->stream));
     if (ones)
       if (int rc = step_graph(s, 1, &s->graph1)) return rc;
-    for (int i = 0; i < n; ++i) DGP_CUDA(cudaGraphLaunch(s->graph, s->stream));
     queued += static_cast<long long>(n) * K;
     if (ones)
       for (; queued < max_steps; ++queued) DGP_CUDA(cudaGraphLaunch(s->graph1, s->stream));
+    // the other graph, for what is left of this run or for the next one
+    if (int rc = step_graph(s, K, &s->graph)) return rc;
+    if (tail)
+      if (int rc = step_graph(s, 1, &s->graph1)) return rc;
     if (int rc = read_ctl(s, &c)) return rc;
     if (c.done == kBadStep) return fail(DGP_ERR_NONPHYSICAL, "time step is not positive and finite");
     if (c.done) break;
@@ -1820,6 +1826,8 @@ int dgp_ensemble_run(dgp_ensemble e, double t0, double tend, double cfl, int max
         for (int i = 0; i < ones; ++i) DGP_CUDA(cudaGraphLaunch(s->graph1, s->stream));
         DGP_CUDA(cudaMemcpyAsync(gpin[g], s->b.gctl, sizeof(TimeCtl), cudaMemcpyDeviceToHost, s->stream));
       }
+    for (dgp_solver s : e->groups)
+      if (int rc = step_graph(s, K, &s->graph)) return rc;
     for (int g = 0; g < G; ++g)
       if (!done[g]) {
         DGP_CUDA(cudaStreamSynchronize(e->groups[g]->stream));

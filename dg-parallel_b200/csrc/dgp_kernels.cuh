@@ -100,7 +100,8 @@ __device__ __forceinline__ size_t slot_index(int e, int s, int j) {
   return ((size_t)(e / K::TE) * K::NS + s) * K::ROWS + (size_t)(e % K::TE) * K::M + j;
 }
 
-constexpr int kBadStep = 2;  // TimeCtl::done: the next time step is not positive and finite
+constexpr int kGraphSteps = 8;  // steps per graph of a run (a power of two)
+constexpr int kBadStep = 2;     // TimeCtl::done: the next time step is not positive and finite
 
 // time-step control that lives in device memory so that a whole run can be
 // captured in a CUDA graph without host round trips
@@ -116,8 +117,8 @@ struct TimeCtl {
   int lts_shift;     // local time stepping: the step is the CFL minimum times 2^lts_shift
   unsigned long long dtmin_bits;  // atomicMin accumulator (positive double bits)
   unsigned int blocks_done;       // completion counter of the reducing kernel
-  int graph_steps;                // steps per graph of a run whose graphs are queued ahead of the
-                                  // host (0: no such run)
+  int one_from;                   // a run whose graphs are queued ahead of the host: the step from
+                                  // which they are of one step each (0: no such run)
   unsigned long long t_mark_ns;   // device clock: run start (whole-launch entry) or
                                   // the moment the instance finished (ensembles)
 };
@@ -589,15 +590,13 @@ __device__ __forceinline__ double ctl_finalize(TimeCtl* c, double dtmin) {
     int N = (int)ceil((c->tend - c->t) / dt);
     dt = (c->tend - c->t) / N;
   }
-  c->dt = dt;
-  c->done = done ? 1 : 0;
-  // a run stops between two graphs (of graph_steps steps, then of one each for
+  // a run stops between two graphs (of kGraphSteps steps, then of one each for
   // what is left under a step limit) where the next step is not positive and
   // finite; the graphs that are queued behind do nothing
-  if (c->graph_steps > 0 && !done && c->steps > 0 && !(dt > 0 && dt < __longlong_as_double(0x7FF0000000000000ll))) {
-    const int left = c->max_steps > 0 ? c->max_steps % c->graph_steps : 0;
-    if (c->steps % c->graph_steps == 0 || (left > 0 && c->steps >= c->max_steps - left)) c->done = kBadStep;
-  }
+  const bool bad = !(dt > 0 && dt < __longlong_as_double(0x7FF0000000000000ll)) && !done && c->one_from > 0 &&
+                   c->steps > 0 && (c->steps % kGraphSteps == 0 || c->steps >= c->one_from);
+  c->dt = dt;
+  c->done = bad ? kBadStep : done ? 1 : 0;
   return dt;
 }
 
