@@ -238,6 +238,7 @@ struct StageArgs {
   int order;
   int p0;          // 1: P0 fallback on (face kernel marks, element kernel consumes marks)
   int ens_tile;    // ensembles: cells per tile of the stage form
+  int late;        // the next kernel of the stream starts late (late_start)
 };
 
 // programmatic dependent launch: the next kernel of the stream may start its
@@ -246,6 +247,22 @@ struct StageArgs {
 // visible.  Without the launch attribute both do nothing.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Where a kernel triggers: at its start, so that the next one's CTAs wait on
+// the SMs with their constant loads done, or late, when its own work is nearly
+// over.  Waiting CTAs hold shared memory and registers, and their first
+// instructions displace the running kernel's.  At the start pays for short
+// kernels alone on the GPU (a step, late / at the start: P0 and P1 of one field
+// 1.03-1.10, P2 1.02-1.04); late pays from P3 on (P3 Euler of 3200 triangles
+// 53 / 57 us, 131072 cells 0.99-1.01), in the limiter's chain of three kernels
+// (P4 Burgers of 8192 and 32768 cells 86 / 104 and 102 / 121 us, P1 37 / 39) and
+// for the groups of an ensemble, whose kernels run in the room left (P1-P4
+// Euler groups of 5408 cells each 124 / 163 us, P4 Burgers of 12800 cells with
+// the limiter 97 / 120).
+template <class K, typename T>
+__device__ __forceinline__ bool late_start(const StageArgs<T>& a) {
+  return K::ORDER >= 3 || a.late;
+}
 
 __device__ __forceinline__ void flag_nonphysical(Status* st, int cell) {
   atomicAdd(&st->nonphysical, 1);
@@ -676,7 +693,7 @@ template <class K>
 __global__ void __launch_bounds__(256) cfl_kernel(const __grid_constant__ StageArgs<typename K::T> a) {
   __shared__ double red[256 / 32];
   __shared__ bool amLast;
-  pdl_trigger();
+  if (!late_start<K>(a)) pdl_trigger();
   pdl_wait();
   if (a.gctl->done) return;
   TimeCtl* c = a.ctl;

@@ -168,8 +168,7 @@ __global__ void __launch_bounds__(128) limit_moments_kernel(LimArgs a) {
   // the CTA's 128 rows are contiguous in the state: they come through shared
   // memory with coalesced loads
   __shared__ double s[128 * NP];
-  pdl_trigger();
-  pdl_wait();
+  pdl_wait();  // (the next kernel starts late)
   if (a.ctl && a.gctl->done) return;
   const size_t R = (size_t)a.E * M;
   const size_t r0 = blockIdx.x * (size_t)128;
@@ -294,8 +293,7 @@ __global__ void __launch_bounds__(128) limit_kernel(LimArgs a) {
   using T = typename K::T;
   constexpr int M = K::M, NP = K::NP, P = K::ORDER, NS = K::NS;
   constexpr int NL = P * (P + 1) / 2;  // moments of degrees 0..p-1
-  pdl_trigger();
-  pdl_wait();
+  pdl_wait();  // (the next kernel starts late)
   if (a.ctl && a.gctl->done) return;
   const size_t R = (size_t)a.E * M;
   const size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x;

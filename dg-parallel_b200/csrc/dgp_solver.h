@@ -153,6 +153,7 @@ inline StageArgs<T> make_args(const DeviceBuffers& b) {
   a.laws = b.laws;
   a.ninst = b.ninst;
   a.ens_tile = b.ens_tile;
+  a.late = b.cell_inst || b.limiter_kind ? 1 : 0;
   a.order = b.order;
   return a;
 }

@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K, TC>::MIN_BLOCKS)
   // last tile with an odd number of values, nor from a base on an odd 8 bytes,
   // a stored state of an odd length), B of the tensor cores.  A bound on the
   // first wait (a.mbar_polls) counts polls from the rows' issue.
-  pdl_trigger();
+  if (!late_start<K>(a)) pdl_trigger();
   const int nrow = min(TS, a.mesh.E - e0);
   const bool bulk = FS::bulk_rows && (nrow * MNP) % 2 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
   const uint32_t rb = bulk ? (uint32_t)(nrow * MNP * 8) : 0u;
@@ -902,6 +902,7 @@ __global__ void __launch_bounds__(K::BLOCK, FusedSmem<K, TC>::MIN_BLOCKS)
     }
   }
 
+  pdl_trigger();  // late at the latest
   // ---- D: gradients + lift + inverse mass + stage combination --------------
   // the FP64 row and u_n (stages 2, 3) come from global memory meanwhile
   double out[NP], u0[NP];
@@ -1074,7 +1075,7 @@ __global__ void __launch_bounds__(kFinalizeThreads) stage_finalize_kernel(
     const __grid_constant__ StageArgs<typename K::T> a, int ntiles) {
   constexpr int NT = kFinalizeThreads;
   __shared__ double red[NT / 32], redd[NT / 32];
-  pdl_trigger();
+  if (!late_start<K>(a)) pdl_trigger();
   pdl_wait();
   if (a.gctl->done) return;
   const double* part = a.partials;
