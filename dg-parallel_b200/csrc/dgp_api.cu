@@ -84,25 +84,26 @@ std::map<std::tuple<int, int, int, int, int, int>, int> g_tune_fused;
 
 // Step times on B200, separate over fused (800 to 524288 triangles, 750 to
 // 384000 tets; brackets: the separate kernels are the default):
-//   triangles P0-P3, and P4 of the linear laws, 1.1-3.1;
-//   P4 of the others in FP64 (0.64, Burgers 0.96) at 3200 cells, 1.0-1.1 at
-//     8192, 1.1-2.0 above; mixed (0.99) at 800, 1.0-1.2 at 3200, 1.2-2.0 above;
-//     the exact Riemann solver in FP64 (0.95) at 16200, 1.06 at 32768, mixed
-//     (0.93) at 3200, 1.09 at 8192: a few tiles expose the fetch of a stage's
-//     unrolled code;
+//   triangles P0-P3, and P4 of the one-field and linear laws, 1.05-3.1, with the
+//     moment limiter 1.1-1.7;
+//   P4 of the Euler law in FP64 (0.75) at 3200 cells, 1.3 at 8192, 1.1-1.4 above,
+//     in an ensemble (0.93) at 8192, 1.1 at 21632; mixed 1.0 at 800, 1.1-1.7 above;
+//     the exact Riemann solver in FP64 (0.76) at 3200, 1.0-1.1 from 8192 on, mixed
+//     (0.94) at 800, 1.0 at 3200, 1.2-1.5 above: a few tiles expose the fetch of a
+//     stage's unrolled code;
 //   P0 of the Euler laws, which leaves the point work a face between two tiles
 //     costs twice: FP64 triangles 1.8-1.9 up to 16200 cells, 1.13 at 65522,
 //     (0.89) at 131072, the exact Riemann solver 0.95 and (0.75), tets 1.6 at
 //     7986, (0.98) at 24576; mixed 1.0 or more but for the exact Riemann solver,
 //     (0.98) at 131072, on tets 1.04 at 48000, (0.89) at 93750;
 //   tets P0, P1 1.1-2.1, P2 0.9 at 8000, 1.4-2.7 above; P3, 20 modes a row, of
-//     the scalar law (0.67) at 7986, 1.1-1.9 above, of Maxwell's in FP64
-//     (0.6-1.0 but for 1.27 at 24576), mixed (0.81) at 3072, 1.5-1.6 above;
+//     the scalar law (0.73) at 7986, 1.1-1.9 above, of Maxwell's in FP64
+//     (0.6-1.1 but for 1.29 at 24576), mixed (0.92) at 3072, 1.5-1.7 above;
 //   the exact Riemann solver on tets: FP64 (0.5-0.8), for about half of the
 //     faces lie between two tiles and are solved twice at ~700 operations a
 //     point; mixed P1 1.0-1.1, (0.98) at 196608, P2 (0.96) at 7986, 1.25 at
 //     24576, 1.06 at 48000, (0.95) at 93750, P3 (0.6-0.95).
-bool fused_default(int law, int flux, int dim, int order, int precision, long long cells) {
+bool fused_default(int law, int flux, int dim, int order, int precision, long long cells, bool ensemble) {
   const bool fp64 = precision == DGP_PRECISION_FP64, riemann = flux == DGP_FLUX_GODUNOV;
   const bool euler = law == DGP_LAW_EULER2D || law == DGP_LAW_EULER3D;
   if (euler && order == 0) {
@@ -110,8 +111,9 @@ bool fused_default(int law, int flux, int dim, int order, int precision, long lo
     return fp64 ? cells < 80000 : !riemann || cells < 120000;
   }
   if (dim == 2) {
-    if (order < 4 || !(euler || law == DGP_LAW_BURGERS2D)) return true;
-    return cells >= (riemann ? (fp64 ? 24000 : 6000) : (fp64 ? 6000 : 2000));
+    if (order < 4 || !euler) return true;
+    if (fp64) return cells >= (ensemble ? 15000 : riemann ? 8000 : 5000);
+    return !riemann || cells >= 2500;
   }
   if (law == DGP_LAW_EULER3D) {
     if (fp64 || order > 2) return false;
@@ -121,10 +123,11 @@ bool fused_default(int law, int flux, int dim, int order, int precision, long lo
   return law == DGP_LAW_SCALAR ? cells >= 16000 : !fp64 && cells >= 5000;
 }
 
-bool tuned_fused(int law, int flux, int dim, int order, int precision, long long cells) {
+bool tuned_fused(int law, int flux, int dim, int order, int precision, long long cells, bool ensemble) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto it = g_tune_fused.find(std::make_tuple(law, flux, dim, order, precision, size_bucket(cells)));
-  return it == g_tune_fused.end() ? fused_default(law, flux, dim, order, precision, cells) : it->second != 0;
+  return it == g_tune_fused.end() ? fused_default(law, flux, dim, order, precision, cells, ensemble)
+                                 : it->second != 0;
 }
 
 void set_tuned_fused(int law, int flux, int dim, int order, int precision, long long cells, bool fused) {
@@ -421,7 +424,8 @@ static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int fie
     nbound += std::count_if(hm.eR.begin(), hm.eR.end(), [](int e) { return e < 0; });
   }
   s->fused_ok = s->ops.fused != nullptr && nbound < (1LL << 26);
-  s->fused = s->fused_ok && (form < 0 ? tuned_fused(s->law, s->flux, dim, s->order, s->precision, cells) : form == 1);
+  s->fused = s->fused_ok && (form < 0 ? tuned_fused(s->law, s->flux, dim, s->order, s->precision, cells, ensemble)
+                                     : form == 1);
   // an ensemble's instances start on the tiles of its form, which it keeps
   const int tile = s->fused ? s->ops.TS : TE;
   if (ensemble) s->fused_ok = s->fused;

@@ -389,8 +389,8 @@ int dgp_backward(dgp_solver s, const double* dJ_duT, double* dJ_du0);
  * each shape both stage forms are timed where the fused stage kernel is built
  * (dgp_set_fused), and the faster is recorded with it (without a record, a
  * default by configuration and size measured on B200: fused, except for the
- * exact Riemann solver on tets, most of P3 on tets, P4 of the nonlinear laws on
- * small meshes and P0 of the Euler laws on large ones).  ms_per_step[3] (may be NULL) gets each shape's best time, -1
+ * exact Riemann solver on tets, most of P3 on tets, P4 of the Euler law on small
+ * meshes and P0 of the Euler laws on large ones).  ms_per_step[3] (may be NULL) gets each shape's best time, -1
  * where not built. */
 int dgp_autotune(dgp_mesh m, dgp_law law, int order, int precision, int limiter, int iters, int* best_block,
                  float* ms_per_step);
