@@ -444,7 +444,6 @@ static int build_solver(dgp_solver s, const std::vector<LawParams>& lps, int fie
   DeviceBuffers& b = s->b;
   b.E = Etot;
   b.dim = dim;
-  b.order = s->order;
   b.M = s->ops.M;
   b.NP = s->ops.NP;
   s->i2f.assign(Etot, -1);

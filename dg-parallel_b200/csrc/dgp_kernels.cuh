@@ -235,10 +235,9 @@ struct StageArgs {
   int ninst;
   int stage;       // 0: RHS only, 1..3: SSP-RK3 stages
   int fuse_cfl;    // stage 3 reduces the next step's dt
-  int order;
+  int late;        // the next kernel of the stream starts late (late_start)
   int p0;          // 1: P0 fallback on (face kernel marks, element kernel consumes marks)
   int ens_tile;    // ensembles: cells per tile of the stage form
-  int late;        // the next kernel of the stream starts late (late_start)
 };
 
 // programmatic dependent launch: the next kernel of the stream may start its

@@ -17,7 +17,7 @@ namespace dgp {
 
 // Device buffers; pointers typed as void* hold the hot-path precision T.
 struct DeviceBuffers {
-  int E = 0, F = 0, NB = 0, order = 0, dim = 0, M = 0, NP = 0;
+  int E = 0, F = 0, NB = 0, dim = 0, M = 0, NP = 0;
   void* jinv = nullptr;
   void* detj = nullptr;
   double* detjd = nullptr;
@@ -154,7 +154,6 @@ inline StageArgs<T> make_args(const DeviceBuffers& b) {
   a.ninst = b.ninst;
   a.ens_tile = b.ens_tile;
   a.late = b.cell_inst || b.limiter_kind ? 1 : 0;
-  a.order = b.order;
   return a;
 }
 
