@@ -25,7 +25,7 @@
 // P3 Euler Roe, 131072 triangles, stages 1 / 2 / 3: FP64 89 / 91 / 110 us
 // (with the tables and rows read from shared memory: 117 / 117 / 142), mixed
 // 59 / 60 / 76 us (94 / 94 / 117).  What bounds it: no unit above 45 % busy
-// (FP64 pipe 35 %, shared memory 40 %); the flux of a face point is a chain of
+// (FP64 pipe 38-40 %, shared memory 40 %); the flux of a face point is a chain of
 // ~50 dependent FP64 operations at 16 resident warps a SM.
 //
 // Laws with a linear flux (advection, Maxwell) need no volume quadrature on

@@ -297,10 +297,11 @@ int dgp_solver_stream(dgp_solver s, void** stream);
 int dgp_profile_kernels(dgp_solver s, int iters, float* ms);
 /* *fused = 1 when each stage runs as one fused stage kernel (faces, volume,
  * lift and the SSP-RK3 update of a tile of cells), 0 when it runs as the face
- * and element kernels (a tile's halo too large for shared memory) */
+ * and element kernels */
 int dgp_solver_fused(dgp_solver s, int* fused);
-/* run the stages as the fused stage kernel (on = 1, the default where it is
- * built) or as the separate face and element kernels (on = 0; also turns off
+/* run the stages as the fused stage kernel (on = 1) or as the separate face and
+ * element kernels (on = 0; the default is the faster form for the configuration
+ * and size, dgp_autotune below measures it; on = 0 also turns off
  * the tensor-core contraction and the rounding probe, which only the fused
  * kernel has); DGP_ERR_UNSUPPORTED when on = 1 and the fused kernel is not
  * built for the solver */
