@@ -1394,9 +1394,13 @@ int dgp_set_p0_fallback(dgp_solver s, int on) {
 
 int dgp_set_tensor_cores(dgp_solver s, int on) {
   if (!s) return fail(DGP_ERR_INVALID, "null solver");
-  if (on && !(s->fused && s->ops.tensor_cores_ok))
+  // where the separate kernels are the default, not the caller's choice, the
+  // fused form takes over
+  const bool fused = s->fused || (s->fused_ok && !s->form_set);
+  if (on && !(fused && s->ops.tensor_cores_ok))
     return fail(DGP_ERR_UNSUPPORTED,
                 "no tensor-core contraction for this solver (mixed form, 128-thread tiles, at most 16 modes)");
+  if (on) s->fused = true;
   s->drop_graphs();
   s->b.tensor_cores = on ? 1 : 0;
   return DGP_OK;
@@ -2038,6 +2042,7 @@ int dgp_set_fused(dgp_solver s, int on) {
   if (!s) return fail(DGP_ERR_INVALID, "null solver");
   if (on && !s->fused_ok)
     return fail(DGP_ERR_UNSUPPORTED, "no fused stage kernel for this solver");
+  s->form_set = true;
   if (on == (s->fused ? 1 : 0)) return DGP_OK;
   DGP_CUDA(cudaSetDevice(s->device));
   s->drop_graphs();

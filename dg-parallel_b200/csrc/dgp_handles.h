@@ -130,6 +130,7 @@ struct dgp_solver_s {
   LtsState lts;                    // local time stepping (off unless enabled)
   std::vector<double> stage_tab;   // host storage of b.htab
   bool fused = false;              // stages run through the fused stage kernel
+  bool form_set = false;           // the caller chose the stage form (dgp_set_fused)
   bool fused_ok = false;           // the fused stage kernel is built for this solver
   bool tr_stale = false;           // the face-point traces (tr) lag the state (the fused
                                    // kernel keeps none; the local time stepping kernels read them)

@@ -85,9 +85,11 @@ extern "C" int dgp_rhs_noalloc(dgp_solver s, const double* dev_state, double t, 
   const size_t state_b = round256(s->state_count() * 8 + 256);
   const size_t ntiles = (static_cast<size_t>(E) + s->ops.TE - 1) / s->ops.TE;
   // the fused stage kernel keeps face data in shared memory: state and RHS
-  // only; the separate kernels also need the face slots and traces
+  // only; the separate kernels also need the face slots and traces, so they run
+  // only where the caller chose them
+  const bool fused = s->fused || (s->fused_ok && !s->form_set);
   const size_t slot_b =
-      s->fused ? 0 : round256(ntiles * s->ops.TE * s->tab.nlf * s->tab.nqf * s->b.M * tsize);
+      fused ? 0 : round256(ntiles * s->ops.TE * s->tab.nlf * s->tab.nqf * s->b.M * tsize);
   const size_t need = 2 * state_b + 2 * slot_b;
   if (need > kScratchBytes)
     return fail(DGP_ERR_INVALID, "dgp_rhs_noalloc: this mesh needs " + std::to_string(need) +
@@ -100,7 +102,7 @@ extern "C" int dgp_rhs_noalloc(dgp_solver s, const double* dev_state, double t, 
   // the separate form's P0 second pass would zero modes of the state copy in
   // place before the element kernel reads it, which the fused kernel does in
   // shared memory only: the fallback applies in the fused form
-  if (!s->fused) b.p0 = 0;
+  if (!fused) b.p0 = 0;
   b.C = p;
   b.slots = p + state_b;
   b.rhs = p + state_b + slot_b;
@@ -114,7 +116,7 @@ extern "C" int dgp_rhs_noalloc(dgp_solver s, const double* dev_state, double t, 
   c.dtmin_bits = 0x7FF0000000000000ull;
   s->h_ctl[0] = c;
   DGP_CUDA(cudaMemcpyAsync(s->b.ctl, &s->h_ctl[0], sizeof(dgp::TimeCtl), cudaMemcpyHostToDevice, s->stream));
-  if (s->fused) {
+  if (fused) {
     const double* C = static_cast<const double*>(b.C);
     s->ops.fused(b, C, C, static_cast<double*>(b.rhs), nullptr, 0, 0.0, 0, s->stream);
   } else {

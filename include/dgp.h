@@ -312,7 +312,7 @@ int dgp_set_fused(dgp_solver s, int on);
  * synchronisation an allocation implies).  dev_state and dev_rhs are device
  * buffers, FP64 [cell][field][mode] in file order, like dgp_rhs's output.  The
  * intermediates (a state and a RHS copy in internal order; with the separate
- * stage form also the face slots and traces) live in a 32 MiB static device
+ * stage form, where dgp_set_fused chose it, also the face slots and traces) live in a 32 MiB static device
  * array that every GPU loading the library holds until exit; meshes that need
  * more return DGP_ERR_INVALID.  The P0 fallback applies in the fused form (as
  * in dgp_rhs) and not in the separate form.

@@ -6,6 +6,7 @@ import pytest
 
 import dgp
 from dgp import meshgen
+from test_zz_no_alloc import rhs_noalloc
 from cases import PULSE3D, SCALAR2D, SCALAR3D, SINE, TM110, VORTEX, rel
 
 pytestmark = pytest.mark.gpu
@@ -88,3 +89,29 @@ def test_autotune_times_both_forms_of_an_ensemble():
         s.project(0.0)
         s.run(0.0, 0.0, 0.1, 4)
         assert rel(e.get_state(i), s.get_state()) < 1e-13
+
+
+def test_default_form_gives_way_where_only_the_fused_one_can():
+    """The separate kernels as a default, not as the caller's choice, refuse
+    nothing: the tensor cores switch to the fused form, and a right-hand side
+    without allocations takes it (145800 cells need 36 MiB of slots otherwise)."""
+    args = (dgp.LAW_EULER3D, dgp.FLUX_GODUNOV, dgp.FIELD_PULSE3D, PULSE3D)
+    s, c = (dgp.Solver(_mesh(3, 4, 3), dgp.Law(*args), 2, dgp.MIXED) for _ in range(2))
+    assert not s.fused
+    s.set_tensor_cores(True)
+    assert s.fused
+    s.run(0.0, 0.0, 0.1, 2)
+    c.set_fused(False)
+    with pytest.raises(dgp.DGPError):
+        c.set_tensor_cores(True)
+    c.run(0.0, 0.0, 0.1, 2)
+    assert rel(s.get_state(), c.get_state()) < 2e-5
+
+    torch = pytest.importorskip("torch")
+    s = dgp.Solver(_mesh(2, 270, 3, box=10.0), dgp.Law(dgp.LAW_EULER2D, dgp.FLUX_ROE, dgp.FIELD_VORTEX, VORTEX), 0)
+    assert not s.fused
+    u = torch.from_numpy(s.get_state().ravel().copy()).cuda()
+    r = torch.full_like(u, float("nan"))
+    torch.cuda.synchronize()
+    assert rhs_noalloc(s, u.data_ptr(), 0.2, r.data_ptr()) == 0
+    assert rel(r.cpu().numpy().reshape(s.shape), s.rhs(0.2)) < 1e-12
